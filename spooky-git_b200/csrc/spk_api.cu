@@ -2148,12 +2148,12 @@ static PassBytes pass_bytes(const spk_ctx* c, bool masked_live = true) {
         // stages 0 and 1 touch the kept modes only; stage 2 also moves the
         // masked modes once (U r, U w)
         b.rhs[0] = nl + 3.0 * c->F * nkxyz * s16;
-        b.rhs[1] = nl + 4.0 * c->F * nkxyz * s16;
+        b.rhs[1] = nl + 3.0 * c->F * nkxyz * s16;
         b.rhs[2] = nl + 3.0 * c->F * nkxyz * s16 + (masked_live ? 2.0 * c->F * (nc - nkxyz) * s16 : 0.0);
         return b;
     }
     b.rhs[0] = nl + 3.0 * c->F * nc * s16;    // U r, U w, S w
-    b.rhs[1] = nl + 4.0 * c->F * nc * s16;    // U r, S r, U w, S w
+    b.rhs[1] = nl + 3.0 * c->F * nc * s16;    // U r, S r, U w (S stays: the scheme's xi_2 = -gamma_2)
     b.rhs[2] = nl + 3.0 * c->F * nc * s16;    // U r, S r, U w
     return b;
 }
