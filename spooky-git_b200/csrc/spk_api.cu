@@ -805,10 +805,6 @@ static RklArgs rkl_args(spk_ctx* c, int stage) {
     for (int v = 0; v < c->nsts; v++) { r.fields[v] = c->sts_fields[v]; r.kind[v] = c->sts_kind[v]; }
     r.nu = c->p.nu; r.nu_m = c->p.nu_m; r.nu_th = c->p.nu_th;
     r.sc = c->sc;
-    r.kxi = c->d_keep; r.kyi = c->d_keep + c->nkx;
-    r.nkx = c->nkx; r.nky = c->nky;
-    r.fd_kzk = FastDiv::make((unsigned)std::max(c->kz_keep, 1));
-    r.fd_nky = FastDiv::make((unsigned)std::max(c->nky, 1));
     return r;
 }
 
@@ -857,11 +853,10 @@ static void record_rkl_cycle(spk_ctx* c) {
             r.nl = c->rA;
             int vslot = 0;
             for (int v = 0; v < c->nsts; v++) if (c->sts_kind[v] == 3) vslot = v;
-            // d_keep is there: nkx, nky, kz_keep > 0 (k = 0 is inside every mask)
-            const int blocks = ew_blocks((size_t)c->nkx * c->nky * c->kz_keep);
+            const FastDiv fz = FastDiv::make((unsigned)c->nzh);
             c->launches++;
-            if (c->fp32) k_rkl_flux<float><<<blocks, 256, 0, c->stream>>>(r, c->U, vslot);
-            else k_rkl_flux<double><<<blocks, 256, 0, c->stream>>>(r, c->U, vslot);
+            if (c->fp32) k_rkl_flux<float><<<ew_blocks(c->nc), 256, 0, c->stream>>>(r, c->U, vslot, fz, FastDiv::make((unsigned)c->ny));
+            else k_rkl_flux<double><<<ew_blocks(c->nc), 256, 0, c->stream>>>(r, c->U, vslot, fz, FastDiv::make((unsigned)c->ny));
         }
     }
 }

@@ -281,9 +281,6 @@ struct RklArgs {
     int nsts; int fields[8]; int kind[8];   // kind: 0 velocity(nu) 1 B(nu_m) 2 th iso(nu_th) 3 th aniso
     double nu, nu_m, nu_th;
     const DevScalars* sc;
-    const int *kxi, *kyi;   // kept x and y indices (the flux update)
-    int nkx, nky;
-    FastDiv fd_kzk, fd_nky;
 };
 
 struct DtArgs {

@@ -1172,29 +1172,29 @@ __global__ void __launch_bounds__(256) k_masked_rk(const __grid_constant__ XfArg
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) k_rkl_flux(const __grid_constant__ RklArgs a, double2* U, int vslot) {
+__global__ void __launch_bounds__(256) k_rkl_flux(const __grid_constant__ RklArgs a, double2* U, int vslot, FastDiv fzh,
+                                                  FastDiv fny) {
     if (a.stage > a.sc->s_rkl) return;
     const double* cf = a.sc->rkl[a.stage];
     const size_t nc = a.g.nc;
-    const int nzh = a.g.nzh, nzs = a.g.nzs, kzk = a.g.kz_keep;
+    const int nzh = a.g.nzh, nzs = a.g.nzs;
     const C2<T>* nl = (const C2<T>*)a.nl;
     double2* Uc = U + (size_t)a.fields[vslot] * nc;
     const double shx = grid_shx(a.g);   // shearing box: the wavevector of the current remap clock
-    // Only the kept modes: outside the 2/3 mask dtheta = 0, and every scheme's
-    // stage is then the identity (RKL2 mu + nu + (1 - mu - nu) = 1, RKL1
-    // mu + nu = 1, STS U + 0).  The pass is bound by the state it moves (four
-    // arrays read, two written in RKL2): 256^3 FP32: 0.116 ms a stage over
-    // every mode, 0.036 over the kept ones (by the step: 43.8 -> 40.6 ms for two).
-    const unsigned total = (unsigned)a.nkx * (unsigned)a.nky * (unsigned)kzk;
-    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const unsigned r1 = a.fd_kzk.div(e), r2 = a.fd_nky.div(r1);
-        const int k = (int)(e - r1 * (unsigned)kzk);
-        const int i = a.kxi[r2], j = a.kyi[r1 - r2 * (unsigned)a.nky];
-        const size_t line = (size_t)i * a.g.ny + j, gi = line * nzh + k, li = line * nzs + k;
-        const double2 q0 = to_d2(nl[li]), q1 = to_d2(nl[a.cs_nl + li]), q2 = to_d2(nl[2 * a.cs_nl + li]);
-        const double kx = a.g.kx[i] + shx * a.g.ky[j], ky = a.g.ky[j], kz = a.g.kz[k];
-        const double2 sq = d2(kx * q0.x + ky * q1.x + kz * q2.x, kx * q0.y + ky * q1.y + kz * q2.y);
-        rkl_update(a, cf, (size_t)vslot * nc, gi, Uc, d2(-sq.y, sq.x));   // i * k.q
+    for (size_t gi = (size_t)blockIdx.x * blockDim.x + threadIdx.x; gi < nc; gi += (size_t)gridDim.x * blockDim.x) {
+        const unsigned line = fzh.div((unsigned)gi);
+        const int k = (int)(gi - (size_t)line * nzh);
+        const unsigned ui = fny.div(line);
+        const int i = (int)ui, j = (int)(line - ui * (unsigned)a.g.ny);
+        double2 dU = d2(0.0, 0.0);
+        if (a.g.mx[i] != 0.0 && a.g.my[j] != 0.0 && a.g.mz[k] != 0.0) {
+            const size_t li = (size_t)line * nzs + k;
+            const double2 q0 = to_d2(nl[li]), q1 = to_d2(nl[a.cs_nl + li]), q2 = to_d2(nl[2 * a.cs_nl + li]);
+            const double kx = a.g.kx[i] + shx * a.g.ky[j], ky = a.g.ky[j], kz = a.g.kz[k];
+            const double2 sq = d2(kx * q0.x + ky * q1.x + kz * q2.x, kx * q0.y + ky * q1.y + kz * q2.y);
+            dU = d2(-sq.y, sq.x);   // i * mask * k.q
+        }
+        rkl_update(a, cf, (size_t)vslot * nc, gi, Uc, dU);
     }
 }
 
