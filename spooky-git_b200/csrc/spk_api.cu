@@ -22,6 +22,7 @@
 
 #include "spk_kernels.cu"
 #include "spk_pass2.cu"
+#include "spk_line.cu"
 #include "spk_closure.cu"
 #include "spk_config.hpp"
 
@@ -218,6 +219,25 @@ static bool make_tmap(const spk_ctx* c, const void* base, int nchan, bool state,
     return r == CUDA_SUCCESS;
 }
 
+// The same of a pass buffer for the warp-owned transforms: swizzled rows of rb
+// bytes, boxes of `rows` positions, columns k >= kext outside the map (loads
+// give zero there, stores write nothing).
+static bool make_line_tmap(const spk_ctx* c, const void* base, int nchan, int axis, int rows, int kext, CUtensorMap* tm,
+                           int rb = 128) {
+    if (!g_encode) return false;
+    const size_t esz = c->fp32 ? 4 : 8, row = (size_t)c->g.nzs;
+    cuuint64_t dims[4] = {(cuuint64_t)(2 * kext), (cuuint64_t)c->ny, (cuuint64_t)c->nx, (cuuint64_t)nchan};
+    cuuint64_t strides[3] = {(cuuint64_t)(2 * row * esz), (cuuint64_t)(2 * row * esz * c->ny),
+                             (cuuint64_t)(2 * row * esz * c->ny * c->nx)};
+    cuuint32_t box[4] = {(cuuint32_t)(rb / esz), 1, 1, 1};
+    box[axis == 0 ? 2 : 1] = (cuuint32_t)rows;
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    return g_encode(tm, c->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
+                    const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    rb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static AxisArgs axis_args(spk_ctx* c, int ax) {
     AxisArgs a;
     memset(&a, 0, sizeof(a));
@@ -361,9 +381,101 @@ static void launch_axis_dir(spk_ctx* c, AxisArgs& a, long total) {
     }
 }
 
+// Kept rows of an axis as tile segments: the prefix, and the suffix from a
+// row that is a multiple of 8 (where the 128-byte swizzle starts again).
+static int kept_segments(const std::vector<double>& mask, int n, LineSeg* seg, int map) {
+    int pre = 0, suf = n;
+    while (pre < n && mask[pre] != 0.0) pre++;
+    while (suf > pre && mask[suf - 1] != 0.0) suf--;
+    suf &= ~7;
+    if (pre == 0 || pre > 256 || n - suf > 256 || suf <= pre) return 0;   // one block (or none): all rows
+    for (int i = pre; i < suf; i++) if (mask[i] != 0.0) return 0;         // not a prefix and a suffix
+    seg[0] = {0, pre, 1, map};
+    seg[1] = {suf, n - suf, n > suf ? 1 : 0, map + 1};
+    return 1 + seg[1].n;
+}
+
+// A pass between pass buffers as k_line; false: not one of its forms.
+template <typename T, int N, int DIR>
+static bool launch_line(spk_ctx* c, const AxisArgs& a, long total) {
+    if constexpr (!line_ok<T, N, 128>()) {
+        return false;
+    } else {
+        if (a.convert || a.defer_stage || a.trim == 1 || !a.in_base || !a.out_base) return false;
+        for (int q = 0; q < a.njobs; q++)
+            if (a.job[q].in_state || a.job[q].hp || a.job[q].deriv > 1) return false;
+        using C = LineCfg<T, N>;
+        LineArgs l;
+        memset(&l, 0, sizeof(l));
+        l.g = a.g; l.plan = a.plan; l.axis = a.axis; l.kcols = a.kcols; l.nb = a.nb; l.njobs = a.njobs;
+        l.in_box_ch = a.in_box_ch; l.out_box_ch = a.out_box_ch;
+        l.outer_filter = a.outer_filter; l.trim = a.trim; l.tr_always = a.tr_always;
+        l.tr_nouter = a.tr_nouter; l.tr_nkb = a.tr_nkb; l.tr_outer = a.tr_outer;
+        l.fd_job = a.fd_job; l.fd_box = a.fd_box; l.fd_kb = a.fd_kb;
+        l.tr_fd_job = a.tr_fd_job; l.tr_fd_box = a.tr_fd_box; l.tr_fd_kb = a.tr_fd_kb;
+        l.scale = a.scale; l.gate = a.gate; l.gate_stage = a.gate_stage; l.err = a.err; l.scs = a.scs;
+        for (int q = 0; q < a.njobs; q++) l.job[q] = {a.job[q].ch, a.job[q].ch_out, a.job[q].deriv};
+        // rows in and out: all of them, or the kept ones (maps 1 and 2)
+        const int rows = N <= 256 ? N : N / 2;
+        const LineSeg all = {0, rows, N / rows, 0};
+        const std::vector<double>& mask = a.axis == 0 ? c->mx : c->my;
+        l.in[0] = all;
+        l.in_trim[0] = all;
+        if (a.trim) kept_segments(mask, N, l.in_trim, 1);
+        l.out = const_cast<void*>(a.out_base);
+        l.out_pre = N; l.out_suf = N;
+        if (a.row_filter) {
+            l.out_pre = 0;
+            while (l.out_pre < N && mask[l.out_pre] != 0.0) l.out_pre++;
+            while (l.out_suf > l.out_pre && mask[l.out_suf - 1] != 0.0) l.out_suf--;
+        }
+        l.out_rows = rows;
+        bool ok = make_line_tmap(c, a.in_base, a.in_nchan, a.axis, rows, a.kcols, &l.map[0]);
+        if (ok && DIR > 0) ok = make_line_tmap(c, a.out_base, a.out_nchan, a.axis, rows, a.kcols, &l.map[3]);
+        for (const LineSeg& s : l.in_trim)
+            if (ok && s.n && s.map) ok = make_line_tmap(c, a.in_base, a.in_nchan, a.axis, s.rows, a.kcols, &l.map[s.map]);
+        if (!ok) {
+            c->err = "internal: cuTensorMapEncodeTiled rejected a pass tensor map";
+            c->sticky = SPK_ERR_CUDA;
+            return true;
+        }
+        // groups per CTA: fewer when the tiles would not reach every SM
+        int ng = C::NG;
+        while (ng > 1 && total < (long)c->num_sms * ng) ng /= 2;
+        const size_t tables = 1024 + (size_t)RegFft<T, N>::TWN * sizeof(C2<T>) + (size_t)((N + 1) & ~1) * sizeof(T) + 2 * 8 * 4 * C::NG;
+        const size_t stage = (size_t)ng * C::G::TILE;
+        const size_t room = (size_t)(227 * 1024) / C::MINB - 1024 - tables;
+        l.nst = (int)std::max<size_t>(2, std::min<size_t>(4, room / stage));
+        if (c->tune_nst >= 2 && c->tune_nst <= 4 && tables + (size_t)c->tune_nst * stage <= (size_t)227 * 1024) l.nst = c->tune_nst;
+        const size_t smem = tables + (size_t)l.nst * stage;
+        const int nthr = ng * C::G::W * 32;
+        allow_full_smem(k_line<T, N, DIR>);
+        int per_sm = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_line<T, N, DIR>, nthr, smem);
+        const int grid = (int)std::min<long>((total + ng - 1) / ng, (long)c->num_sms * std::max(per_sm, 1));
+        c->launches++;
+        k_line<T, N, DIR><<<grid, nthr, smem, c->stream>>>(l);
+        return true;
+    }
+}
+
+template <typename T, int DIR>
+static bool launch_line_dir(spk_ctx* c, const AxisArgs& a, long total) {
+    switch (a.plan.n) {
+#define SPK_LINE_CASE(n) case n: return launch_line<T, n, DIR>(c, a, total);
+        SPK_FOR_EACH_LENGTH(SPK_LINE_CASE)
+#undef SPK_LINE_CASE
+        default: return false;
+    }
+}
+
 template <typename T>
 static void launch_axis(spk_ctx* c, AxisArgs& a, int dir) {
     const int nouter = a.axis == 0 ? c->ny : c->nx;
+    const int kt0 = a.kt;
+    for (int form = 0; form < 2; form++) {
+    // k_line's 128-byte tiles first, then k_axis2's own tile width
+    a.kt = form == 0 ? (int)(128 / csize(c)) : kt0;
     const int nkb = (a.kcols + a.kt - 1) / a.kt;
     const long total = (long)a.njobs * a.nb * nouter * nkb;
     if (total <= 0) return;
@@ -390,8 +502,13 @@ static void launch_axis(spk_ctx* c, AxisArgs& a, int dir) {
         a.tr_fd_box = FastDiv::make((unsigned)(a.tr_nouter * a.tr_nkb));
         a.tr_fd_job = FastDiv::make((unsigned)(a.nb * a.tr_nouter * a.tr_nkb));
     }
+    if (form == 0) {
+        if (dir > 0 ? launch_line_dir<T, +1>(c, a, total) : launch_line_dir<T, -1>(c, a, total)) return;
+        continue;
+    }
     if (dir > 0) launch_axis_dir<T, +1>(c, a, total);
     else launch_axis_dir<T, -1>(c, a, total);
+    }
 }
 
 static void axis(spk_ctx* c, AxisArgs& a, int dir) {
@@ -524,6 +641,14 @@ static void add_job(spk_ctx* c, AxisArgs& a, const void* in, void* out, int nch,
         a.box_rows = d;
     }
     if (in_state && c->fp32) a.convert = 1;
+    // the arrays, if the jobs of the pass share them
+    const void* obase = nullptr;
+    int onchan = 0, och0 = 0;
+    locate(c, out, false, &obase, &onchan, &och0);
+    const bool same = a.njobs == 0 || (a.in_base == base && a.out_base == obase);
+    a.in_base = same && !in_state ? base : nullptr;
+    a.out_base = same ? obase : nullptr;
+    a.in_nchan = nchan; a.out_nchan = onchan;
     a.in_box_ch = in_state ? c->F : buf_channels(c, base);
     if (c->nb > 1 && (base == c->rA || base == c->rB || base == c->user_U)) {
         c->bad_job = true;
@@ -539,6 +664,7 @@ static void add_job(spk_ctx* c, AxisArgs& a, const void* in, void* out, int nch,
         }
         j.out = (char*)out + (size_t)q * chan_bytes(c);
         j.ch = ch0 + q;
+        j.ch_out = och0 + q;
         j.in_state = in_state;
         j.deriv = deriv;
     }

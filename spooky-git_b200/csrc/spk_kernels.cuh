@@ -153,7 +153,7 @@ struct AxisJob {
                     // 2 k of the outer index, 3 kz of the column
     int defer_grp;  // deferred masked modes: 1 velocity (nu), 2 magnetic field (nu_m), 0 none
     int hp;         // keep only |k|^2 > AxisArgs::hp_k2 (the small scales of the closure's variant 2)
-    int pad_;
+    int ch_out;     // channel of the output in AxisArgs::out_base
 };
 
 struct AxisArgs {
@@ -191,6 +191,9 @@ struct AxisArgs {
     const int* tr_outer;
     int tr_always;          // enumerate the kept tiles regardless of the flag (outer-filtered x forward)
     FastDiv tr_fd_job, tr_fd_box, tr_fd_kb;
+    // the arrays of the jobs (host side; a pass between two of them may run as k_line)
+    const void *in_base, *out_base;
+    int in_nchan, out_nchan;
     int njobs;
     AxisJob job[SPK_MAXJOBS];
 };
