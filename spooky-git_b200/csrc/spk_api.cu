@@ -23,6 +23,7 @@
 #include "spk_kernels.cu"
 #include "spk_pass2.cu"
 #include "spk_line.cu"
+#include "spk_xrhs.cu"
 #include "spk_closure.cu"
 #include "spk_config.hpp"
 
@@ -893,6 +894,69 @@ static XfArgs xf_args(spk_ctx* c, double2* U, int mode, bool clean) {
     return x;
 }
 
+// ---------------------------------------------------------------------------
+// x forward + RHS + x inverse of stages 0 and 1 (k_xrhs)
+// ---------------------------------------------------------------------------
+// The steps it covers: deferred masked modes and trimmed inverse passes (HD
+// and MHD), no closure (its x inverse has gradient channels), an x length
+// whose tile fits.
+template <typename T>
+static bool xrhs_length(int n) {
+    switch (n) {
+#define SPK_XR_CASE(m) case m: return xr_ok<T, m>();
+        SPK_FOR_EACH_LENGTH(SPK_XR_CASE)
+#undef SPK_XR_CASE
+        default: return false;
+    }
+}
+static bool xrhs_fused(const spk_ctx* c) {
+    return c->trim_now && !c->closure_on && (c->fp32 ? xrhs_length<float>(c->nx) : xrhs_length<double>(c->nx));
+}
+
+template <typename T, int N>
+static void launch_xrhs(spk_ctx* c, const XfArgs& x) {
+    if constexpr (xr_ok<T, N>()) {
+        constexpr int RB = xr_rb<T, N>();
+        using G = Line<T, N, RB>;
+        XrArgs a;
+        memset(&a, 0, sizeof(a));
+        a.x = x;
+        a.in_box_ch = a.out_box_ch = c->nbuf_ch;
+        a.err = &c->sc->err;
+        const int nchan = c->nbuf_ch * c->nb;
+        if (!make_line_tmap(c, c->bufB, nchan, 0, N, c->kz_keep, &a.in, RB) ||
+            !make_line_tmap(c, c->bufA, nchan, 0, N, c->nzh, &a.out, RB)) {
+            c->err = "internal: cuTensorMapEncodeTiled rejected a pass tensor map";
+            c->sticky = SPK_ERR_CUDA;
+            return;
+        }
+        a.ch_T = c->out_T; a.ch_E = c->out_E; a.ch_u = c->ch_u; a.ch_b = c->ch_b;
+        a.scale = 1.0 / ((double)c->nx * (double)c->ny * (double)c->nz);
+        const int nkb = (c->nzh + G::KT - 1) / G::KT, nkbk = (c->kz_keep + G::KT - 1) / G::KT;
+        a.fd_kb = FastDiv::make((unsigned)nkb); a.fd_outer = FastDiv::make((unsigned)c->ny);
+        a.tr_fd_kb = FastDiv::make((unsigned)nkbk); a.tr_fd_outer = FastDiv::make((unsigned)c->nky);
+        using F = RegFft<T, N>;
+        const size_t smem = 1024 + (size_t)5 * G::TILE + (size_t)((F::TWN + 1) & ~1) * sizeof(C2<T>) + (size_t)8 * N +
+                            (size_t)((N + 7) & ~7) + 16;
+        static_assert(N <= 256, "a TMA box holds every row");
+        allow_full_smem(k_xrhs<T, N>);
+        int per_sm = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_xrhs<T, N>, 256, smem);
+        const long total = (long)(c->p.mhd ? 2 : 1) * c->nb * c->ny * nkb;
+        c->launches++;
+        k_xrhs<T, N><<<(int)std::min<long>(total, (long)c->num_sms * std::max(per_sm, 1)), 256, smem, c->stream>>>(a);
+    }
+}
+
+static void xrhs(spk_ctx* c, const XfArgs& x) {
+    switch (c->nx) {
+#define SPK_XR_CASE(m) case m: if (c->fp32) launch_xrhs<float, m>(c, x); else launch_xrhs<double, m>(c, x); break;
+        SPK_FOR_EACH_LENGTH(SPK_XR_CASE)
+#undef SPK_XR_CASE
+        default: break;
+    }
+}
+
 static DtArgs dt_args(spk_ctx* c, bool advance) {
     DtArgs d;
     memset(&d, 0, sizeof(d));
@@ -1063,7 +1127,9 @@ static void record_step_body(spk_ctx* c, int parity, bool rk_only) {
     for (int s = 0; s < nst; s++) {
         const bool first = s == 0 && !rk_only;
         c->stage_csh = (shear && !euler) ? csh[s] : 0.0;
-        pass_x_inverse(c, c->U, true, euler ? 0 : s);
+        // stages 1 and 2 of a fused step: the previous stage's k_xrhs left the x inverse
+        const bool fused = !euler && !rk_only && xrhs_fused(c);
+        if (s == 0 || !fused) pass_x_inverse(c, c->U, true, euler ? 0 : s);
         pass_y_inverse(c, true);
         if (first) {
             if (sts_before) {
@@ -1085,7 +1151,8 @@ static void record_step_body(spk_ctx* c, int parity, bool rk_only) {
         pass_y_forward(c, c->nout, c->bufA, c->bufB);
         // the last stage cleans the new u and B: CleanFieldDivergence of the next step
         XfArgs x = xf_args(c, c->U, euler ? XM_EULER : s, s == nst - 1 && !rk_only && !shear);
-        xfwd(c, x);
+        if (fused && s < nst - 1) xrhs(c, x);
+        else xfwd(c, x);
     }
     c->stage_csh = 0.0;
     if (shear) {

@@ -1,18 +1,21 @@
-"""The strided-axis passes on warp-owned transforms (k_line), at the
-lengths where its tiles and masks change, against the CPU FP64 oracle.
-Tolerances as in test_gpu_parity.py.
+"""The strided-axis passes on warp-owned transforms (k_line) and the fused
+x forward + RHS + x inverse of RK3 stages 0 and 1 (k_xrhs), at the lengths
+where their tiles, masks and box kinds change, against the CPU FP64 oracle.
+Tolerances as in test_gpu_parity.py; a few steps of the FP32 form stay
+within 1e-6 of the oracle (one RHS of 2e-5 times dt |dU| / |U| < 1e-2 a stage).
 """
 import numpy as np
 import pytest
 
 import oracle as O
 from fields import random_solenoidal, to_spectral
-from spooky_b200 import Context
+from spooky_b200 import Context, Ensemble
 from spooky_b200.initial import masked_noise_state
 from spooky_b200.params import SPK_FORM_FP32, SPK_FORM_PLAIN, default_params
 
 pytestmark = pytest.mark.gpu
 FORMS = [SPK_FORM_PLAIN, SPK_FORM_FP32]
+TOL_STEP = {SPK_FORM_PLAIN: 1e-12, SPK_FORM_FP32: 1e-6}
 TOL_RHS = {SPK_FORM_PLAIN: 1e-12, SPK_FORM_FP32: 2e-5}
 
 
@@ -36,6 +39,54 @@ def state(p, seed, outside):
     if p.antialiasing:
         U = U * O.Oracle(p).kgrid()[1]
     return masked_noise_state(p, U, rel=0.2, seed=seed) if outside else U
+
+
+def check_steps(p, U, nsteps, tol):
+    o = O.Oracle(p)
+    o.set_state(U)
+    o.step(nsteps)
+    ctx = Context(p)
+    ctx.set_state(U)
+    ctx.advance(nsteps)
+    ctx.synchronize()
+    assert rel_l2(ctx.get_state(), o.get_state()) < tol
+
+
+# every x length k_xrhs covers; 24 y rows and 9 kz columns leave ragged tiles
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("outside", [False, True])
+@pytest.mark.parametrize("nx", [24, 32, 48, 64, 96, 128, 192, 256])
+def test_fused_stage_matches_oracle(nx, outside, form):
+    p = params((nx, 24, 16), nx % 3 == 0 or nx >= 128, form)
+    check_steps(p, state(p, 5, outside), 3, TOL_STEP[form])
+
+
+# several k blocks, the last one partial; and no dealiasing (every mode kept)
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("antialiasing", [1, 0])
+def test_fused_stage_many_columns(antialiasing, form):
+    p = params((64, 16, 96), 1, form, antialiasing=antialiasing)
+    check_steps(p, state(p, 6, False), 2, TOL_STEP[form])
+
+
+# boxes with and without content outside the mask in one group: the fused
+# pass takes both kinds of box in one launch
+@pytest.mark.parametrize("form", FORMS)
+def test_fused_stage_mixed_group(form):
+    ps = [params((48, 24, 32), 1, form) for _ in range(3)]
+    for p, nu in zip(ps, (1e-2, 5e-3, 2e-3)):
+        p.nu = nu
+    Us = [state(p, 7 + i, i == 1) for i, p in enumerate(ps)]
+    ens = Ensemble(ps)
+    for b, U in zip(ens.boxes, Us):
+        b.set_state(U)
+    ens.advance(3)
+    ens.synchronize()
+    for p, U, b in zip(ps, Us, ens.boxes):
+        o = O.Oracle(p)
+        o.set_state(U)
+        o.step(3)
+        assert rel_l2(b.get_state(), o.get_state()) < TOL_STEP[form]
 
 
 # every length k_line covers along y, with more than one k block
