@@ -533,37 +533,44 @@ static void axis(spk_ctx* c, AxisArgs& a, int dir) {
 
 template <typename T, int N>
 static void launch_zpass_ln(spk_ctx* c, ZArgs& z, int nin_all) {
-    const int nthr = 128;
-    const int slots = std::max(1, nthr / RegFft<T, N>::TPC);
+    constexpr int TPC = RegFft<T, N>::TPC;
     const long nlines = (long)c->nx * c->ny;
-    const int npin = (nin_all + 1) / 2, npout = (z.nout + 1) / 2;
     const int gen = z.closure == 3 ? 3 : (z.closure ? 2 : ((z.derive_gz != 0 || z.mode == ZM_TO_REAL || z.shear_part) ? 1 : 0));
-    const int max_ctas = gen == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4;   // the kernel's launch bounds
-    auto need = [&](int lines) {
-        return zsmem_layout(N, RegFft<T, N>::TWN, (int)sizeof(C2<T>), z.nin, nin_all, npout, lines, c->g.nzs,
+    const int max_ctas = zpass_minb<T>(gen);   // the kernel's launch bounds
+    auto need = [&](int lines, int nt) {
+        const int slots = std::max(1, nt / TPC);
+        return zsmem_layout(N, RegFft<T, N>::TWN, (int)sizeof(C2<T>), z.nin, nin_all, zpass_pairs(z.nout, lines, z.xline), lines, c->g.nzs,
                             slots, z.closure == 3 ? C3_ZBYTES / 4 : (z.closure ? CL_NP : 0),
-                            zpass_alias(gen, RegFft<T, N>::NS, npin, npout, lines, slots),
+                            zpass_alias(gen, RegFft<T, N>::NS, zpass_pairs(nin_all, lines, z.xline), zpass_pairs(z.nout, lines, z.xline), slots),
                             (gen == 1 && z.load_breal && zpass_stage_b<T, N>()) ? 3 : 0).total;
     };
-    // lines per CTA: best (busy transform slots) x (resident CTAs per SM, <= 4)
-    auto rounds = [&](long n) { return (n + slots - 1) / slots; };
-    int L = 1;
+    // Lines per CTA, and 96 or 128 threads (4 or 3 warps): the most lines per
+    // transform slot of the rounds, times the resident warps (by shared memory,
+    // the kernel's launch bounds and the lines there are).  An odd channel's lines pair up across
+    // a CTA's lines: an even number of lines, so that the pairs (and the bits)
+    // do not depend on the choice (nx ny is a multiple of 4).
+    const bool even = z.xline && ((nin_all | z.nout) & 1) && need(2, 128) <= (size_t)227 * 1024;
+    int tz = c->tune_zl + (even ? c->tune_zl & 1 : 0);   // the caller's lines, where they fit
+    if (tz > nlines || need(tz, 128) > (size_t)227 * 1024 || (c->nb > 1 && tz > 0 && nlines % tz != 0)) tz = 0;
+    int L = 1, nthr = 128;
     double best = -1.0;
-    for (int cand = 1; cand <= 64 && cand <= nlines; cand *= 2) {
-        if (c->nb > 1 && nlines % cand != 0) break;   // a CTA's lines stay inside one box
-        const size_t sm = need(cand);
-        if (sm > (size_t)227 * 1024) break;
-        const long work = (long)(npin + npout) * cand;
-        const long cap = (rounds((long)npin * cand) + rounds((long)npout * cand)) * slots;
-        const double util = (double)work / (double)std::max<long>(cap, 1);
-        const int ctas = (int)std::min<size_t>((size_t)max_ctas, (size_t)(233472 / (sm + 1024)));
-        const double score = util * ctas;
-        if (score >= best) { best = score; L = cand; }
+    for (int nt = 128; nt >= 96; nt -= 32) {
+        if (nt % TPC != 0 || (nt < 128 && z.closure)) continue;
+        const long slots = std::max(1, nt / TPC);
+        auto cap = [&](long n) { return (n + slots - 1) / slots * slots; };
+        for (int cand = tz > 0 ? tz : 1; cand <= (tz > 0 ? tz : std::min(64L, nlines)); cand = cand < 16 ? cand + 1 : 2 * cand) {
+            if (even && (cand & 1)) continue;
+            if (c->nb > 1 && nlines % cand != 0) continue;   // a CTA's lines stay inside one box
+            const size_t sm = need(cand, nt);
+            if (sm > (size_t)227 * 1024) break;
+            const long r = cap(zpass_pairs(nin_all, cand, z.xline)) + cap(zpass_pairs(z.nout, cand, z.xline));
+            const int ctas = (int)std::min<size_t>((size_t)(max_ctas * 128 / nt), (size_t)(233472 / (sm + 1024)));
+            const double fill = std::min(1.0, (double)nlines * c->nb / cand / ((double)c->num_sms * ctas));
+            const double score = (double)cand / (double)std::max<long>(r, 1) * ctas * nt * fill;
+            if (score > best || (score == best && nt == nthr)) { best = score; L = cand; nthr = nt; }
+        }
     }
-    if (c->tune_zl > 0 && c->tune_zl <= nlines && need(c->tune_zl) <= (size_t)227 * 1024 &&
-        (c->nb == 1 || nlines % c->tune_zl == 0))
-        L = c->tune_zl;
-    const size_t smem = need(L);
+    const size_t smem = need(L, nthr);
     if (smem > (size_t)227 * 1024) {
         c->err = "internal: z pass tile exceeds shared memory";
         c->sticky = SPK_ERR_UNSUPPORTED;
@@ -772,6 +779,7 @@ static ZArgs z_args(spk_ctx* c) {
     z.nb = c->nb;
     z.in_box = z.out_box = (size_t)c->nbuf_ch * c->g.ncs;
     z.scs = c->sc;
+    z.xline = c->p.boussinesq ? 0 : 1;
     return z;
 }
 

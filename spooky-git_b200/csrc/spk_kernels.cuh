@@ -237,6 +237,7 @@ struct ZArgs {
     // diagnostics (general path only): 1 -- the symmetric matrix v_i v_j of
     // the vector at ch_u, components xx xy xz; 2 -- components yy yz zz
     int shear_part;
+    int xline;              // an odd channel pairs with itself on the next line (zpass_pairs)
 };
 
 enum XMode { XM_RK0 = 0, XM_RK1 = 1, XM_RK2 = 2, XM_EULER = 3, XM_DFIELD = 4 };

@@ -349,14 +349,24 @@ struct ZSmem { size_t tw, zero, junk, area, real, xb, cw, bre, total; };
 // and at least two FFT stages keeps its exchange slots in the input/product
 // area: every slot has loaded its legs before the first exchange barrier (a
 // one-stage transform has no such barrier before its stores to the slots)
-__host__ __device__ inline bool zpass_alias(int gen, int nstages, int npin, int npout, int lines, int slots) {
-    return gen == 0 && nstages >= 2 && npin * lines <= slots && npout * lines <= slots;
+__host__ __device__ inline bool zpass_alias(int gen, int nstages, int ninv, int nfw, int slots) {
+    return gen <= 1 && nstages >= 2 && ninv <= slots && nfw <= slots;
+}
+// Complex transforms of a CTA of `lines` lines with nch real channels: the
+// channels of a line pair up; the last of an odd number is a transform of its
+// own, or with xline pairs with the same channel of the next line (the last
+// line of an odd number stays alone).  HD makes 4 transforms a line that way
+// (3 channels in, 5 out) instead of 5: 512^3 FP32 2.56 -> 2.05 ms a pass,
+// 256^3 FP32 0.256 -> 0.213, FP64 0.533 -> 0.433.  Boussinesq contexts keep the pairs within the line: the conduction
+// cycle carries a changed FP32 rounding through every stage after it.
+__host__ __device__ inline int zpass_pairs(int nch, int lines, int xline) {
+    return (nch / 2) * lines + ((nch & 1) ? (xline ? (lines + 1) / 2 : lines) : 0);
 }
 // Exchange slots of the z pass pad one element per 128-byte row of complex
 // elements (16 in FP32, 8 in FP64), which keeps the exchanges of the
 // register FFT free of bank conflicts in both precisions.
 __host__ __device__ constexpr int zpass_xblock(int csz) { return 128 / csz; }
-__host__ __device__ inline ZSmem zsmem_layout(int n, int twn, int csz, int nin, int nin_all, int npout, int lines,
+__host__ __device__ inline ZSmem zsmem_layout(int n, int twn, int csz, int nin, int nin_all, int nfw, int lines,
                                               int nzs, int slots, int ncw, bool alias, int nbre = 0) {
     ZSmem z;
     const int rs = n + 16, xs = n + n / zpass_xblock(csz);
@@ -364,7 +374,7 @@ __host__ __device__ inline ZSmem zsmem_layout(int n, int twn, int csz, int nin, 
     z.zero = align16(z.tw + (size_t)twn * csz);              // a zero half spectrum (missing pair partner)
     z.junk = align16(z.zero + (size_t)nzs * csz);            // a real row that idle transforms write
     z.area = align16(z.junk + (size_t)rs * (csz / 2));
-    const size_t raw = (size_t)nin * lines * nzs * csz, prod = (size_t)npout * lines * n * csz;
+    const size_t raw = (size_t)nin * lines * nzs * csz, prod = (size_t)nfw * n * csz;
     const size_t xbs = (size_t)slots * xs * csz;
     size_t area = raw > prod ? raw : prod;
     if (alias && xbs > area) area = xbs;
@@ -386,13 +396,18 @@ __host__ __device__ inline ZSmem zsmem_layout(int n, int twn, int csz, int nin, 
 // when a line's bytes keep every bulk copy 16-byte aligned.
 template <typename T, int N> __host__ __device__ constexpr bool zpass_stage_b() { return (N * sizeof(T)) % 16 == 0; }
 
+// CTAs of 128 threads per SM the z pass is compiled for
+template <typename T> __host__ __device__ constexpr int zpass_minb(int gen) {
+    return gen == 0 ? (sizeof(T) == 4 ? 6 : 5) : (gen == 1 && sizeof(T) == 4 ? 5 : 4);
+}
+
 // GEN: 0 -- every input channel is a plain half spectrum; 1 -- derived
 // gradient channels or the to-real output (the general path); 2 -- the
 // general path with the learned closure (its own instantiation, so that the
 // MLP's registers do not weigh on the others); 3 -- the same with the
 // closure's tensor network (variant 3).
 template <typename T, int N, int GEN>
-__global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) k_zpass2(const __grid_constant__ ZArgs a) {
+__global__ void __launch_bounds__(128, zpass_minb<T>(GEN)) k_zpass2(const __grid_constant__ ZArgs a) {
     using F = RegFft<T, N>;
     constexpr int LTPC = F::LTPC, TPC = F::TPC;
     constexpr int RS = N + 16;            // real rows: consecutive lines start 16 words apart in bank
@@ -410,16 +425,17 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
     const int nin = a.nin;
     const int nder0 = nin + (a.derive_gz == 1 ? 1 : 0);   // first closure d/dz channel
     const int nin_all = nder0 + (GEN >= 2 ? a.zder_n : 0);
-    const int npin = (nin_all + 1) / 2, npout = (a.nout + 1) / 2;
+    const int ninv = zpass_pairs(nin_all, L, a.xline), nfw = zpass_pairs(a.nout, L, a.xline);   // transforms
+    const int nfull_in = (nin_all / 2) * L, nfull_out = (a.nout / 2) * L;      // of them within a line
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int slots = nthr >> LTPC;
     const int sigma = tid >> LTPC, q = tid & (TPC - 1);
     const int sigma_w = (tid & ~31) >> LTPC;   // the lowest slot of this warp (warp-uniform)
     const bool clos = GEN >= 2 && a.closure;
-    const bool alias = zpass_alias(GEN, F::NS, npin, npout, L, slots);
+    const bool alias = zpass_alias(GEN, F::NS, ninv, nfw, slots);
     // flux mode: the CTA's real B lines arrive with the inputs, off the point loop's path
     const bool stage_b = GEN == 1 && zpass_stage_b<T, N>() && a.load_breal;
-    const ZSmem lay = zsmem_layout(N, F::TWN, (int)sizeof(C2<T>), nin, nin_all, npout, L, nzs, slots,
+    const ZSmem lay = zsmem_layout(N, F::TWN, (int)sizeof(C2<T>), nin, nin_all, nfw, L, nzs, slots,
                                    clos ? (GEN == 3 ? C3_ZBYTES / 4 : CL_NP) : 0, alias, stage_b ? 3 : 0);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);
     C2<T>* tw = reinterpret_cast<C2<T>*>(smem_raw + lay.tw);
@@ -487,65 +503,75 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
     auto xaddr = [&](int Lx) { return xb + (size_t)sigma * XS + padb<XB>(Lx); };
     C2<T> r[F::E];
 
+    // Transform tau: channel chA of line lA with channel chB of line lB (chB =
+    // -1: no partner; a line past the CTA's last holds no data).
+    struct Pair { int chA, lA, chB, lB; };
+    auto pair_of = [&](int tau, int nch, int nfull) {
+        Pair x;
+        if (tau < nfull) {
+            const int p = tau / L;
+            x.chA = 2 * p; x.chB = 2 * p + 1;
+            x.lA = x.lB = tau - p * L;
+        } else {
+            x.chA = nch - 1;
+            x.lA = (a.xline ? 2 : 1) * (tau - nfull); x.lB = x.lA + 1;
+            x.chB = a.xline && x.lB < nl ? nch - 1 : -1;
+        }
+        return x;
+    };
+
     // 2. inverse transforms of the input pairs
-    const int ninv = npin * L;
     for (int base = 0; base < ninv; base += slots) {
         const int tau = base + sigma;
         const bool valid = tau < ninv;
-        const int p = valid ? tau / L : 0, l = valid ? tau - p * L : 0;
+        const Pair x = pair_of(valid ? tau : 0, nin_all, nfull_in);
         // false: no slot of this warp has a transform, and the warp skips the math
         const bool act = base + sigma_w < ninv;
-        const C2<T>* pa = raw + (size_t)(2 * p * L + l) * nzs;
-        const C2<T>* pb = 2 * p + 1 < nin ? pa + (size_t)L * nzs : zrow;
-        auto chv = [&](int ch, int k) -> C2<T> {
-            if (k >= kzk) return mk<T>((T)0, (T)0);
-            if (ch < nin) {
-                C2<T> v = raw[((size_t)ch * L + l) * nzs + k];
-                if (a.derive_gz == 2 && ch == a.ch_th) {
-                    const T kz = (T)a.g.kz[k];
-                    v = mk<T>(-kz * v.y, kz * v.x);
+        // a channel's source row in the input area, and whether it enters as its d/dz
+        auto source = [&](int ch, int l, bool& dz) -> const C2<T>* {
+            dz = false;
+            if (ch < 0) return zrow;
+            if constexpr (GEN != 0) {
+                if (a.derive_gz == 2 && ch == a.ch_th) dz = true;
+                if (ch >= nin) {
+                    dz = true;
+                    ch = ch < nder0 ? a.ch_th : a.zder_src[ch - nder0];   // theta; closure: u [and B]
                 }
-                return v;
             }
-            if (ch == nin && a.derive_gz == 1) {
-                const C2<T> th = raw[((size_t)a.ch_th * L + l) * nzs + k];
-                const T kz = (T)a.g.kz[k];
-                return mk<T>(-kz * th.y, kz * th.x);
-            }
-            if (ch >= nder0 && ch < nin_all) {   // closure: d/dz of u [and B]
-                const C2<T> x = raw[((size_t)a.zder_src[ch - nder0] * L + l) * nzs + k];
-                const T kz = (T)a.g.kz[k];
-                return mk<T>(-kz * x.y, kz * x.x);
-            }
-            return mk<T>((T)0, (T)0);
+            return raw + (size_t)(ch * L + l) * nzs;
         };
+        bool dza, dzb;
+        const C2<T>* pa = source(x.chA, x.lA, dza);
+        const C2<T>* pb = source(x.chB, x.lB, dzb);
         if (act) regfft_load<T, N, +1>(r, q, [&](int n) -> C2<T> {
             constexpr int NH = N >> 1;
             const int k = n <= NH ? n : N - n;
             C2<T> A, B;
-            if constexpr (GEN == 0) {
-                const C2<T> zz = mk<T>((T)0, (T)0);
-                A = k < kzk ? pa[k] : zz;
-                B = k < kzk ? pb[k] : zz;
-            } else {
-                A = chv(2 * p, k);
-                B = chv(2 * p + 1, k);
+            const C2<T> zz = mk<T>((T)0, (T)0);
+            A = k < kzk ? pa[k] : zz;
+            B = k < kzk ? pb[k] : zz;
+            if constexpr (GEN != 0) {
+                if (dza || dzb) {
+                    const T kz = (T)a.g.kz[k];
+                    if (dza) A = mk<T>(-kz * A.y, kz * A.x);
+                    if (dzb) B = mk<T>(-kz * B.y, kz * B.x);
+                }
             }
             if (n == 0 || n == NH) return mk<T>(A.x, B.x);
             if (n < NH) return mk<T>(A.x - B.y, A.y + B.x);
             return mk<T>(A.x + B.y, B.x - A.y);
         });
-        // an idle transform (and the missing partner of an odd last pair) writes the junk row
-        T* pr0 = valid ? real + (size_t)(2 * p * L + l) * RS : junk;
-        T* pr1 = (valid && 2 * p + 1 < nin_all) ? pr0 + LRS : junk;
-        const bool to_real = GEN != 0 && a.mode == ZM_TO_REAL && valid && l < nl;
+        // an idle transform (and a missing partner) writes the junk row
+        T* pr0 = valid ? real + (size_t)(x.chA * L + x.lA) * RS : junk;
+        T* pr1 = (valid && x.chB >= 0) ? real + (size_t)(x.chB * L + x.lB) * RS : junk;
+        const bool to_real = GEN != 0 && a.mode == ZM_TO_REAL && valid;
         regfft_run<T, N, +1, false, XB>(r, q, tw, xaddr, [&](int z, C2<T> v) {
             pr0[z] = v.x;
             pr1[z] = v.y;
             if (GEN != 0 && to_real) {
-                const size_t line = (size_t)(line0 + l);
-                if (2 * p < nin) a.real_out[((size_t)(2 * p) * nlines + line) * N + z] = (double)v.x;
-                if (2 * p + 1 < nin) a.real_out[((size_t)(2 * p + 1) * nlines + line) * N + z] = (double)v.y;
+                if (x.chA < nin && x.lA < nl) a.real_out[((size_t)x.chA * nlines + line0 + x.lA) * N + z] = (double)v.x;
+                if (x.chB >= 0 && x.chB < nin && x.lB < nl)
+                    a.real_out[((size_t)x.chB * nlines + line0 + x.lB) * N + z] = (double)v.y;
             }
         }, act);
     }
@@ -561,6 +587,17 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
         int bad = 0;
         const T third = (T)(1.0 / 3.0);
         const size_t pstride = (size_t)L * N * 2;   // scalars between product pairs
+        const bool odd = (a.nout & 1) != 0;
+        // the last channel of an odd number at point z of line l: with xline
+        // half of the pair of lines (l, l + 1), zero for a line without data;
+        // zero in the place of a missing partner
+        auto put_odd = [&](int l, int z, T v) {
+            T* po = prodT + (size_t)(nfull_out + (a.xline ? l >> 1 : l)) * 2 * N;
+            auto at = [&](int h) -> T& { return po[PLANES ? h * N + z : 2 * z + h]; };
+            const int h = a.xline ? l & 1 : 0;
+            at(h) = l < nl ? v : (T)0;
+            if (h == 0 && (!a.xline || l + 1 >= L)) at(1) = (T)0;
+        };
         // the closure's gradient components of the point at fr (variant 2: all nine
         // of each field from ch_dx; else d/dx, d/dy and the z-derivative channels)
         auto grads = [&](const T* fr, float* A, float* G) {
@@ -597,7 +634,7 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
         auto hdmhd_loop = [&](auto mhd_c) {
             constexpr bool MHD = decltype(mhd_c)::value;
             const int cu = a.ch_u * LRS, cb = MHD ? a.ch_b * LRS : 0;
-            const bool dmax = a.do_max != 0, odd = (a.nout & 1) != 0;
+            const bool dmax = a.do_max != 0;
             for (int e = tid; e < L * N; e += nthr) {
                 const int l = (int)((unsigned)e / (unsigned)N), z = e - l * N;
                 const T* fr = real + (size_t)l * RS + z;
@@ -619,7 +656,7 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
                     put(1, ux * uy);
                     put(2, ux * uz);
                     put(3, (-ux * ux + (T)2.0 * uy * uy - uz * uz) * third);
-                    put(4, uy * uz);
+                    put_odd(l, z, uy * uz);   // HD: five channels
                 } else {
                     put(0, ((T)2.0 * ux * ux - uy * uy - uz * uz - (T)2.0 * bx * bx + by * by + bz * bz) * third);
                     put(1, ux * uy - bx * by);
@@ -630,7 +667,6 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
                     put(6, bx * uz - bz * ux + (T)0.f);
                     put(7, -bx * uy + by * ux + (T)0.f);
                 }
-                if (odd) put(a.nout, (T)0);
             }
         };
         // The anisotropic heat flux of an RKL2 stage (ZM_RKL_FLUX with the real
@@ -645,7 +681,6 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
         } else if (flux) {
             const int cgx = a.ch_gx * LRS, cgy = a.ch_gy * LRS, cgz = a.ch_th * LRS;
             const int sd = a.sd;
-            const bool odd = (a.nout & 1) != 0;
             const T chi = (T)a.chi, W = (T)a.omegaT2;
             for (int e = tid; e < L * N; e += nthr) {
                 const int l = (int)((unsigned)e / (unsigned)N), z = e - l * N;
@@ -664,8 +699,7 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
                 const T bs = sd == 0 ? bx : (sd == 1 ? by : bz);
                 put(0, chi * bx * (bgt + W * bs) / b2);
                 put(1, chi * by * (bgt + W * bs) / b2);
-                put(2, chi * bz * (bgt + W * bs) / b2);
-                if (odd) put(a.nout, (T)0);
+                put_odd(l, z, chi * bz * (bgt + W * bs) / b2);   // three channels
             }
         } else
         for (int e0 = 0; e0 < L * N; e0 += EPC) {
@@ -726,7 +760,10 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
             if (a.derive_gz == 1) gz = fr[nin * LRS];
             else if (a.derive_gz == 2) gz = fr[a.ch_th * LRS];
             T* pp = prodT + (PLANES ? (size_t)l * 2 * N + z : ((size_t)l * N + z) * 2);
-            auto put = [&](int ch, T v) { pp[(size_t)(ch >> 1) * pstride + (ch & 1) * CS] = v; };
+            auto put = [&](int ch, T v) {
+                if (odd && ch == a.nout - 1) put_odd(l, z, v);
+                else pp[(size_t)(ch >> 1) * pstride + (ch & 1) * CS] = v;
+            };
             int qc = 0;
             // learned closure: -2 nu_t S into the stress, -eta_t J into the EMF
             float ctau[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, cemf[3] = {0.f, 0.f, 0.f};
@@ -755,22 +792,22 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
             }
             if (a.mode == ZM_PRODUCTS) {
                 if (a.hydro) {
+                    T p[5];
                     if (!a.mhd) {
-                        put(0, ((T)2.0 * ux * ux - uy * uy - uz * uz) * third);
-                        put(1, ux * uy);
-                        put(2, ux * uz);
-                        put(3, (-ux * ux + (T)2.0 * uy * uy - uz * uz) * third);
-                        put(4, uy * uz);
+                        p[0] = ((T)2.0 * ux * ux - uy * uy - uz * uz) * third;
+                        p[1] = ux * uy;
+                        p[2] = ux * uz;
+                        p[3] = (-ux * ux + (T)2.0 * uy * uy - uz * uz) * third;
+                        p[4] = uy * uz;
                     } else {
-                        put(0, ((T)2.0 * ux * ux - uy * uy - uz * uz - (T)2.0 * bx * bx + by * by + bz * bz) * third);
-                        put(1, ux * uy - bx * by);
-                        put(2, ux * uz - bx * bz);
-                        put(3, (-ux * ux + (T)2.0 * uy * uy - uz * uz + bx * bx - (T)2.0 * by * by + bz * bz) * third);
-                        put(4, uy * uz - by * bz);
+                        p[0] = ((T)2.0 * ux * ux - uy * uy - uz * uz - (T)2.0 * bx * bx + by * by + bz * bz) * third;
+                        p[1] = ux * uy - bx * by;
+                        p[2] = ux * uz - bx * bz;
+                        p[3] = (-ux * ux + (T)2.0 * uy * uy - uz * uz + bx * bx - (T)2.0 * by * by + bz * bz) * third;
+                        p[4] = uy * uz - by * bz;
                     }
-                    if (clos)
 #pragma unroll
-                        for (int r = 0; r < 5; r++) pp[(size_t)(r >> 1) * pstride + (r & 1) * CS] += (T)ctau[r];
+                    for (int r = 0; r < 5; r++) put(r, clos ? p[r] + (T)ctau[r] : p[r]);
                     qc = 5;
                 }
                 if (a.mhd) {
@@ -794,7 +831,6 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
                 put(qc + 2, chi * bz * (bgt + W * bs) / b2);
                 qc += 3;
             }
-            if (a.nout & 1) put(a.nout, (T)0);
         }
         if constexpr (GEN == 3) {
             if (clos) __syncthreads();   // the chunk's outputs are read before the next chunk's inputs
@@ -827,15 +863,13 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
     C2<T>* out = (C2<T>*)a.out + (size_t)box * a.out_box;
     const T half = (T)0.5;
     const int lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
-    const int nfw = npout * L;
     for (int base = 0; base < nfw; base += slots) {
         if (base > 0) __syncthreads();   // the previous round's unpack has read the exchange slots
         const int tau = base + sigma;
-        const bool valid = tau < nfw;
-        const int p = valid ? tau / L : 0, l = valid ? tau - p * L : 0;
-        const T* pp = prodT + (size_t)(p * L + l) * 2 * N;
-        // (forward rounds: FP64 only; in FP32 the branches cost more than they save, measured)
-        const bool act = sizeof(T) == 4 || base + sigma_w < nfw;
+        const T* pp = prodT + (size_t)(tau < nfw ? tau : 0) * 2 * N;
+        // (forward rounds in FP32 with several transforms a warp: the branches
+        // cost more than they save, measured)
+        const bool act = (sizeof(T) == 4 && TPC < 32) || base + sigma_w < nfw;
         if (act) regfft_load<T, N, -1>(r, q, [&](int z) -> C2<T> {
             if constexpr (PLANES) return mk<T>(pp[z], pp[N + z]);
             else return reinterpret_cast<const C2<T>*>(pp)[z];
@@ -845,13 +879,12 @@ __global__ void __launch_bounds__(128, GEN == 0 ? (sizeof(T) == 4 ? 6 : 5) : 4) 
         for (int s2 = warp; s2 < slots; s2 += nwarp) {
             const int tau2 = base + s2;
             if (tau2 >= nfw) break;
-            const int p2 = tau2 / L, l2 = tau2 - p2 * L;
-            if (l2 >= nl) continue;
+            const Pair x = pair_of(tau2, a.nout, nfull_out);
+            if (x.lA >= nl) continue;
             const C2<T>* Z = xb + (size_t)s2 * XS;
-            const size_t off0 = (size_t)(line0 + l2) * nzs;
-            C2<T>* o0 = out + (size_t)(2 * p2) * a.cs_out + off0;
-            C2<T>* o1 = out + (size_t)(2 * p2 + 1) * a.cs_out + off0;
-            const bool two = 2 * p2 + 1 < a.nout;
+            C2<T>* o0 = out + (size_t)x.chA * a.cs_out + (size_t)(line0 + x.lA) * nzs;
+            C2<T>* o1 = out + (size_t)x.chB * a.cs_out + (size_t)(line0 + x.lB) * nzs;
+            const bool two = x.chB >= 0;
             for (int k = lane; k < kk; k += 32) {
                 const C2<T> zk = Z[padb<XB>(k)], zm = Z[padb<XB>(k ? N - k : 0)];
                 o0[k] = mk<T>(half * (zk.x + zm.x), half * (zk.y - zm.y));
