@@ -2354,7 +2354,7 @@ static PassBytes pass_bytes(const spk_ctx* c, bool masked_live = true) {
         return b;
     }
     b.rhs[0] = nl + 3.0 * c->F * nc * s16;    // U r, U w, S w
-    b.rhs[1] = nl + 3.0 * c->F * nc * s16;    // U r, S r, U w (S stays: the scheme's xi_2 = -gamma_2)
+    b.rhs[1] = nl + (c->p.boussinesq ? 4.0 : 3.0) * c->F * nc * s16;   // U r, S r, U w (and S w: rk_value)
     b.rhs[2] = nl + 3.0 * c->F * nc * s16;    // U r, S r, U w
     return b;
 }

@@ -908,7 +908,7 @@ __global__ void __launch_bounds__(128, zpass_minb<T>(GEN)) k_zpass2(const __grid
 // ---------------------------------------------------------------------------
 // New state value of one mode given its RK scratch value S (read up front).
 __device__ __forceinline__ double2 rk_value(const XfArgs& a, size_t gi, double2 X, double2 S, double2 R, double dt) {
-    const double g0 = 8.0 / 15.0, g1 = 5.0 / 12.0, g2 = 3.0 / 4.0, x0 = -17.0 / 60.0;
+    const double g0 = 8.0 / 15.0, g1 = 5.0 / 12.0, g2 = 3.0 / 4.0, x0 = -17.0 / 60.0, x1 = -5.0 / 12.0;
     switch (a.mode) {
         case XM_RK0: {
             // U1 = U + g0 dt R, then S = U1 + x0 dt R (the second axpyComplex
@@ -920,9 +920,13 @@ __device__ __forceinline__ double2 rk_value(const XfArgs& a, size_t gi, double2 
         }
         case XM_RK1: {
             // the scheme's S = U2 + x1 dt R has x1 = -g1, so it is the S that
-            // was read: the store (one array of the stage's four) is left out
-            const double bu = g1 * dt;
-            return d2(1.0 * S.x + bu * R.x, 1.0 * S.y + bu * R.y);
+            // was read, but for rounding: the store (one array of the stage's
+            // four) is left out.  Boussinesq contexts keep it: their conduction
+            // cycle carries a last bit of the state through every FP32 stage.
+            const double bu = g1 * dt, bs = x1 * dt;
+            const double2 Un = d2(1.0 * S.x + bu * R.x, 1.0 * S.y + bu * R.y);
+            if (a.bous) a.S[gi] = d2(1.0 * Un.x + bs * R.x, 1.0 * Un.y + bs * R.y);
+            return Un;
         }
         case XM_RK2: {
             const double bu = g2 * dt;
