@@ -191,30 +191,51 @@ __global__ void k_masked_flag(DevScalars* scs) {
 // f1 f2 over the grid (twoFieldCorrelation).  Per-CTA shared-memory
 // histograms, then atomics into out (summation order varies).
 // ---------------------------------------------------------------------------
-__global__ void k_spectrum(DevGrid g, const double2* U1, const double2* U2, int nbins, double dk, double inv_n,
-                           double* out) {
+// A warp's modes are consecutive in kz, so equal shells lie side by side: each
+// run is summed by shuffles and its last lane adds it to the histogram.  Bound
+// by instruction issue (the shell's FP64 square root and divide, 40 us of
+// reads at 256^3); one add per mode, and 64-bit index divisions, cost 84 us
+// against 63 here.
+__global__ void __launch_bounds__(512) k_spectrum(DevGrid g, const double2* U1, const double2* U2, int nbins, double dk,
+                                                  double inv_n, double* out, FastDiv fzh, FastDiv fny) {
     extern __shared__ double hist[];
     for (int m = threadIdx.x; m < nbins; m += blockDim.x) hist[m] = 0.0;
     __syncthreads();
-    const size_t nc = g.nc;
+    const unsigned nc = (unsigned)g.nc;   // below 2^31 for every supported size
     const int nzl = g.nz / 2;   // Nyquist plane index
     const double shx = grid_shx(g);
+    const unsigned lane = threadIdx.x & 31;
     double tot = 0.0;
-    for (size_t gi = (size_t)blockIdx.x * blockDim.x + threadIdx.x; gi < nc; gi += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(gi % g.nzh);
-        const size_t r = gi / g.nzh;
-        const int j = (int)(r % g.ny), i = (int)(r / g.ny);
-        const double2 a = U1[gi], b = U2[gi];
-        const double pr = (a.x * inv_n) * (b.x * inv_n) + (a.y * inv_n) * (b.y * inv_n);
-        const double p = k > 0 ? 2.0 * pr : pr;
-        tot += (k > 0 && k != nzl) ? 2.0 * pr : pr;
-        const double kx = g.kx[i] + shx * g.ky[j], ky = g.ky[j], kz = g.kz[k];
-        const int m = (int)(sqrt(kx * kx + ky * ky + kz * kz) / dk + 0.5);
-        if (m < nbins) atomicAdd(&hist[m], p);
+    for (unsigned g0 = blockIdx.x * blockDim.x; g0 < nc; g0 += gridDim.x * blockDim.x) {   // whole warps
+        const unsigned gi = g0 + threadIdx.x;
+        double p = 0.0;
+        int m = -1;
+        if (gi < nc) {
+            const unsigned r = fzh.div(gi);
+            const int k = (int)(gi - r * (unsigned)g.nzh);
+            const unsigned ui = fny.div(r);
+            const int i = (int)ui, j = (int)(r - ui * (unsigned)g.ny);
+            const double2 a = U1[gi], b = U2[gi];
+            const double pr = (a.x * inv_n) * (b.x * inv_n) + (a.y * inv_n) * (b.y * inv_n);
+            p = k > 0 ? 2.0 * pr : pr;
+            tot += (k > 0 && k != nzl) ? 2.0 * pr : pr;
+            const double kx = g.kx[i] + shx * g.ky[j], ky = g.ky[j], kz = g.kz[k];
+            m = (int)(sqrt(kx * kx + ky * ky + kz * kz) / dk + 0.5);
+            if (m >= nbins) m = -1;
+        }
+        const int mp = __shfl_up_sync(0xffffffffu, m, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || mp != m);
+        const unsigned first = 31u - __clz(heads & (0xffffffffu >> (31u - lane)));   // the run's first lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double v = __shfl_up_sync(0xffffffffu, p, o);
+            if (lane >= first + o) p += v;
+        }
+        if (m >= 0 && (lane == 31 || ((heads >> (lane + 1)) & 1u))) atomicAdd(&hist[m], p);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&out[nbins], tot);
+    if (lane == 0) atomicAdd(&out[nbins], tot);
     __syncthreads();
     for (int m = threadIdx.x; m < nbins; m += blockDim.x)
         if (hist[m] != 0.0) atomicAdd(&out[m], hist[m]);

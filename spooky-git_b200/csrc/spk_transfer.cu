@@ -227,15 +227,9 @@ extern "C" int spk_transfer_spectra(spk_ctx* c, const char* kind_name, double* o
     if (ncomp) *ncomp = nt;
     if (nbins) *nbins = c->nbins;
     if (deltak) *deltak = c->deltak;
-    const double inv_n = 1.0 / ((double)c->nx * (double)c->ny * (double)c->nz);
-    const int grid = (int)std::min<size_t>((c->nc + 255) / 256, (size_t)c->num_sms * 8);
     std::vector<double> h((size_t)c->nbins + 1);
     for (int q = 0; q < nt; q++) {
-        CK(cudaMemsetAsync(c->d_spec, 0, sizeof(double) * (size_t)(c->nbins + 1), c->stream));
-        k_spectrum<<<grid, 256, sizeof(double) * (size_t)c->nbins, c->stream>>>(
-            c->g, c->U + (size_t)(f0 + q) * c->nc, c->S + (size_t)q * c->nc, c->nbins, c->deltak, inv_n, c->d_spec);
-        c->launches++;
-        rc = launch_status(c);
+        rc = launch_spectrum(c, c->U + (size_t)(f0 + q) * c->nc, c->S + (size_t)q * c->nc);
         if (rc) return rc;
         CK(cudaMemcpyAsync(h.data(), c->d_spec, sizeof(double) * (size_t)(c->nbins + 1), cudaMemcpyDeviceToHost,
                            c->stream));
