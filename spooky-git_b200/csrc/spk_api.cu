@@ -365,7 +365,13 @@ static void launch_axis_conv(spk_ctx* c, AxisArgs& a, long total) {
     if constexpr (sizeof(T) == 4 && DIR > 0) {
         if (a.convert) { launch_axis_ln<T, N, DIR, true>(c, a, total); return; }
     }
-    launch_axis_ln<T, N, DIR, false>(c, a, total);
+    // k_line takes every forward pass of the lengths it covers
+    if constexpr (DIR > 0 || !line_ok<T, N, 128>()) {
+        launch_axis_ln<T, N, DIR, false>(c, a, total);
+    } else {
+        c->err = "internal: a forward axis pass without its kernel";
+        c->sticky = SPK_ERR_CUDA;
+    }
 }
 
 // Every transform length the register FFT covers (2^k and 3*2^k).
@@ -917,9 +923,10 @@ static bool xrhs_length(int n) {
         default: return false;
     }
 }
-static bool xrhs_fused(const spk_ctx* c) {
-    return c->trim_now && !c->closure_on && (c->fp32 ? xrhs_length<float>(c->nx) : xrhs_length<double>(c->nx));
+static bool xrhs_able(const spk_ctx* c) {
+    return c->defer && c->d_keep && !c->closure_on && (c->fp32 ? xrhs_length<float>(c->nx) : xrhs_length<double>(c->nx));
 }
+static bool xrhs_fused(const spk_ctx* c) { return c->trim_now && xrhs_able(c); }
 
 template <typename T, int N>
 static void launch_xrhs(spk_ctx* c, const XfArgs& x) {
@@ -2315,7 +2322,7 @@ extern "C" const char* spk_last_error(const spk_ctx* c) {
 // ---------------------------------------------------------------------------
 // accounting and per-pass timing
 // ---------------------------------------------------------------------------
-struct PassBytes { double x_inv, y_inv, z, y_fwd, x_fwd, rhs[3]; };
+struct PassBytes { double x_inv, y_inv, z, y_fwd, x_fwd, rhs[3], xr; };   // xr: x forward + RHS + x inverse of a stage
 
 // Algorithmic HBM bytes of each pass: every array the pass must read or
 // write, once; products only where the 2/3 mask keeps them.
@@ -2345,6 +2352,10 @@ static PassBytes pass_bytes(const spk_ctx* c, bool masked_live = true) {
     b.y_fwd = c->nout * nkz * b_t + c->nout * nkyz * b_t;
     b.x_fwd = c->nout * nkyz * b_t + c->nout * nkxyz * b_t;
     const double nl = c->nout * nkxyz * b_t;
+    // products in, state (three of U r, S r, U w, S w), x inverse out; the
+    // masked modes of a live state pass through
+    b.xr = c->nout * nkyz * b_t + 3.0 * c->F * nkxyz * s16 +
+           (masked_live ? c->F * (nc - nkxyz) * s16 + c->F * nc * b_t : c->F * nkyz * b_t);
     if (c->defer) {
         // stages 0 and 1 touch the kept modes only; stage 2 also moves the
         // masked modes once (U r, U w)
@@ -2386,7 +2397,8 @@ extern "C" int spk_step_info(spk_ctx* c, int* kps, double* bytes) {
                 for (int b2 = 0; b2 < c->nb; b2++) live = live || c->h_sc[b2].masked_live != 0;
             }
             const PassBytes b = pass_bytes(c, live);
-            *bytes = 3.0 * (b.x_inv + b.y_inv + b.z + b.y_fwd + b.x_fwd) + b.rhs[0] + b.rhs[1] + b.rhs[2];
+            *bytes = 3.0 * (b.y_inv + b.z + b.y_fwd) + b.x_inv + b.x_fwd + b.rhs[2] +
+                     (xrhs_able(c) ? 2.0 * b.xr : 2.0 * (b.x_inv + b.x_fwd) + b.rhs[0] + b.rhs[1]);
         }
     }
     return SPK_OK;
@@ -2410,9 +2422,12 @@ extern "C" int spk_profile_passes(spk_ctx* c, int reps, spk_pass_stat_t* out, in
     TrimScope ts(c);   // time the passes as a step runs them
     // with deferred masked modes the RHS of stages 0-1 (kept modes) and of
     // stage 2 (kept modes + the step's masked modes) are timed apart
-    const char* names[7] = {"x_inverse", "y_inverse", "z_products", "y_forward", "x_forward", "rhs_rk", "rhs_rk_01"};
-    const double bytes[7] = {pb.x_inv, pb.y_inv, pb.z, pb.y_fwd, pb.x_fwd, pb.rhs[2], pb.rhs[1]};
-    const int npass = c->defer ? 7 : 6;
+    // (rhs_rk_01 runs in a step only where the fused pass does not)
+    const bool fused = xrhs_able(c);
+    const char* names[8] = {"x_inverse", "y_inverse", "z_products", "y_forward", "x_forward", "rhs_rk", "rhs_rk_01", "x_fwd_rhs_x_inv"};
+    const double bytes[8] = {pb.x_inv, pb.y_inv, pb.z, pb.y_fwd, pb.x_fwd, pb.rhs[2], pb.rhs[1], pb.xr};
+    const int per_step[8] = {fused ? 1 : 3, 3, 3, 3, fused ? 1 : 3, c->defer ? 1 : 3, fused ? 0 : 2, 2};
+    const int npass = fused ? 8 : (c->defer ? 7 : 6);
     int n = 0;
     // one warm pipeline so every buffer holds stage data
     pass_x_inverse(c, c->U, true, 2);
@@ -2430,7 +2445,8 @@ extern "C" int spk_profile_passes(spk_ctx* c, int reps, spk_pass_stat_t* out, in
                 case 3: pass_y_forward(c, c->nout, c->bufA, c->bufB); break;
                 case 4: pass_x_forward(c); break;
                 case 5: { XfArgs x = xf_args(c, c->U, XM_RK2, false); rhs(c, x); } break;
-                default: { XfArgs x = xf_args(c, c->U, XM_RK1, false); rhs(c, x); } break;
+                case 6: { XfArgs x = xf_args(c, c->U, XM_RK1, false); rhs(c, x); } break;
+                default: { XfArgs x = xf_args(c, c->U, XM_RK1, false); xrhs(c, x); } break;
             }
         }
         CK(cudaEventRecord(e1, c->stream));
@@ -2441,7 +2457,7 @@ extern "C" int spk_profile_passes(spk_ctx* c, int reps, spk_pass_stat_t* out, in
         strncpy(out[n].name, names[k], sizeof(out[n].name) - 1);
         out[n].ms = ms / reps;
         out[n].bytes = bytes[k];
-        out[n].launches_per_step = (c->defer && k == 5) ? 1 : (k == 6 ? 2 : 3);
+        out[n].launches_per_step = per_step[k];
         n++;
     }
     cudaEventDestroy(e0);
