@@ -193,7 +193,7 @@ __global__ void k_masked_flag(DevScalars* scs) {
 // ---------------------------------------------------------------------------
 // A warp's modes are consecutive in kz, so equal shells lie side by side: each
 // run is summed by shuffles and its last lane adds it to the histogram.  Bound
-// by instruction issue (the shell's FP64 square root and divide, 40 us of
+// by instruction issue (the shell's FP64 square root and divide; 20 us of
 // reads at 256^3); one add per mode, and 64-bit index divisions, cost 84 us
 // against 63 here.
 __global__ void __launch_bounds__(512) k_spectrum(DevGrid g, const double2* U1, const double2* U2, int nbins, double dk,
