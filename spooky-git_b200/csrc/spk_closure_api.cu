@@ -200,7 +200,10 @@ extern "C" int spk_spectrum(spk_ctx* c, int f1, int f2, double* out, int max_bin
     if (nbins) *nbins = c->nbins;
     if (deltak) *deltak = c->deltak;
     if (c->nbins < 1) return fail(c, SPK_ERR_UNSUPPORTED, "no spectral bins for this grid");
-    if (!out && !total) return launch_status(c);   // the sizes alone
+    if (!out && !total) {   // the sizes alone
+        CK(cudaStreamSynchronize(c->stream));
+        return launch_status(c);
+    }
     int rc = launch_spectrum(c, c->U + (size_t)f1 * c->nc, c->U + (size_t)f2 * c->nc);
     if (rc) return rc;
     std::vector<double> h((size_t)c->nbins + 1);
