@@ -467,7 +467,10 @@ __global__ void k_reset_max(DevScalars* sc) {
 // Stage 1 of RKL1 keeps U in Uc1 only: the reference's copies to Uc0 and
 // dU0 are never read by that scheme.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void rkl_update(const RklArgs& a, const double* c, size_t off, size_t gi, double2* Uc, double2 dU) {
+// zero: dU = 0 in every stage of the cycle (a mode that the flux does not
+// reach); its dU0 is neither written nor read, and enters as the zero it is.
+__device__ __forceinline__ void rkl_update(const RklArgs& a, const double* c, size_t off, size_t gi, double2* Uc, double2 dU,
+                                           bool zero = false) {
     double2* Uc0 = a.Uc0 + off;
     double2* Uc1 = a.Uc1 + off;
     double2* dU0 = a.dU0 + off;
@@ -475,7 +478,10 @@ __device__ __forceinline__ void rkl_update(const RklArgs& a, const double* c, si
     if (a.sts_alg == STS_ALG_STS) {
         Uc[gi] = d2(1.0 * U.x + c[2] * dU.x, 1.0 * U.y + c[2] * dU.y);
     } else if (a.stage == 1) {
-        if (a.sts_alg == STS_ALG_RKL2) { Uc0[gi] = U; dU0[gi] = dU; }
+        if (a.sts_alg == STS_ALG_RKL2) {
+            Uc0[gi] = U;
+            if (!zero) dU0[gi] = dU;
+        }
         Uc1[gi] = U;
         Uc[gi] = d2(1.0 * U.x + c[2] * dU.x, 1.0 * U.y + c[2] * dU.y);
     } else if (a.sts_alg == STS_ALG_RKL1) {
@@ -484,7 +490,7 @@ __device__ __forceinline__ void rkl_update(const RklArgs& a, const double* c, si
         Uc1[gi] = U;
         Uc[gi] = d2(Y.x + c[2] * dU.x, Y.y + c[2] * dU.y);
     } else {
-        const double2 U1 = Uc1[gi], U0 = Uc0[gi], D0 = dU0[gi];
+        const double2 U1 = Uc1[gi], U0 = Uc0[gi], D0 = zero ? d2(0.0, 0.0) : dU0[gi];
         const double2 Y = d2(c[0] * U.x + c[1] * U1.x, c[0] * U.y + c[1] * U1.y);
         Uc1[gi] = U;
         Uc[gi] = d2(Y.x + c[4] * U0.x + c[2] * dU.x + c[3] * D0.x, Y.y + c[4] * U0.y + c[2] * dU.y + c[3] * D0.y);

@@ -1224,14 +1224,17 @@ __global__ void __launch_bounds__(256) k_rkl_flux(const __grid_constant__ RklArg
         const unsigned ui = fny.div(line);
         const int i = (int)ui, j = (int)(line - ui * (unsigned)a.g.ny);
         double2 dU = d2(0.0, 0.0);
-        if (a.g.mx[i] != 0.0 && a.g.my[j] != 0.0 && a.g.mz[k] != 0.0) {
+        // (the pass moves at the copy bandwidth: dU0 of the masked 70% of the
+        // modes left out is a ninth of its bytes, 256^3 FP32 0.115 -> 0.099 ms)
+        const bool kept = a.g.mx[i] != 0.0 && a.g.my[j] != 0.0 && a.g.mz[k] != 0.0;
+        if (kept) {
             const size_t li = (size_t)line * nzs + k;
             const double2 q0 = to_d2(nl[li]), q1 = to_d2(nl[a.cs_nl + li]), q2 = to_d2(nl[2 * a.cs_nl + li]);
             const double kx = a.g.kx[i] + shx * a.g.ky[j], ky = a.g.ky[j], kz = a.g.kz[k];
             const double2 sq = d2(kx * q0.x + ky * q1.x + kz * q2.x, kx * q0.y + ky * q1.y + kz * q2.y);
             dU = d2(-sq.y, sq.x);   // i * mask * k.q
         }
-        rkl_update(a, cf, (size_t)vslot * nc, gi, Uc, dU);
+        rkl_update(a, cf, (size_t)vslot * nc, gi, Uc, dU, !kept);
     }
 }
 
