@@ -449,7 +449,8 @@ static bool launch_line(spk_ctx* c, const AxisArgs& a, long total) {
         // groups per CTA: fewer when the tiles would not reach every SM
         int ng = C::NG;
         while (ng > 1 && total < (long)c->num_sms * ng) ng /= 2;
-        const size_t tables = 1024 + (size_t)RegFft<T, N>::TWN * sizeof(C2<T>) + (size_t)((N + 1) & ~1) * sizeof(T) + 2 * 8 * 4 * C::NG;
+        const size_t tables = 1024 + (size_t)RegFft<T, N>::TWN * sizeof(C2<T>) + (size_t)((N + 1) & ~1) * sizeof(T) +
+                              (2 * 8 * 4 + 8) * C::NG;   // ... barriers and load counts
         const size_t stage = (size_t)ng * C::G::TILE;
         const size_t room = (size_t)(227 * 1024) / C::MINB - 1024 - tables;
         l.nst = (int)std::max<size_t>(2, std::min<size_t>(4, room / stage));

@@ -27,6 +27,7 @@
 // touching its tiles, still meets its barriers, and the pass ends with
 // DevScalars.err = 2.
 #include "spk_line.cuh"
+#include "spk_ring.cuh"
 
 namespace spk {
 
@@ -88,6 +89,8 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
     // per stage: loaded (TMA bytes), then read out by every warp of the group
     uint64_t* bar = reinterpret_cast<uint64_t*>(kax + ((N + 1) & ~1)) + 2 * grp * nst;
     uint64_t* empty = bar + nst;
+    // the group's loads so far (its first thread's; in shared memory, off the registers)
+    int* issued = reinterpret_cast<int*>(reinterpret_cast<uint64_t*>(kax + ((N + 1) & ~1)) + 2 * ng * nst) + grp;
 
     // a pass whose boxes all have no masked content walks only the tiles it keeps
     bool all_clear = a.trim != 0;
@@ -125,6 +128,7 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
     };
     auto issue = [&](int t, int s) {   // the group's first thread
         const Where x = where(t);
+        ++*issued;
         if (x.skip) { mbar_expect_tx(&bar[s], 0); return; }
         const LineSeg* seg = x.clear ? a.in_trim : a.in;
         mbar_expect_tx(&bar[s], (uint32_t)((seg[0].rows * seg[0].n + seg[1].rows * seg[1].n) * 128));
@@ -134,6 +138,7 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
     };
 
     if (lead) {
+        *issued = 0;
         for (int s = 0; s < nst; s++) { mbar_init(&bar[s], 1); mbar_init(&empty[s], W); }
         fence_mbar_init();
         for (int s = 0; s < nst; s++)
@@ -227,9 +232,11 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
     if (TOUT && lead) bulk_wait<0>();
     if (dead) {
         if (lane == 0) atomicExch(a.err, 2);
-        // bounded drain of the loads in flight
+        // bounded drain of the loads in flight: the group has walked its tiles
+        // to the end without loading, so they are counted by what went out
         if (lead)
-            for (int s = 0; s < nst; s++) mbar_wait(&bar[s], (uint32_t)(((it + s) / nst) & 1), SPK_WAIT_ITERS);
+            for (int j = ring_first_pending(*issued, nst); j < *issued; j++)
+                mbar_wait(&bar[ring_stage(j, nst)], ring_parity(j, nst), SPK_WAIT_ITERS);
     }
 }
 
