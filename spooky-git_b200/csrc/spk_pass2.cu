@@ -14,6 +14,7 @@
 #include "spk_regfft.cuh"
 #include "spk_closure.cuh"
 #include "spk_closure3.cuh"
+#include "spk_ring.cuh"
 
 namespace spk {
 
@@ -316,7 +317,10 @@ __global__ void __launch_bounds__(256, axis_minb<T, N>()) k_axis2(const __grid_c
     if (aborted) {
         if (tid == 0) {
             atomicExch(a.err, 2);
-            for (int s = 0; s < NST; s++) mbar_wait(&bar[s], (uint32_t)(((i + s) / NST) & 1), SPK_WAIT_ITERS);
+            // bounded drain: the loads of tiles i .. i + NST - 1, as far as this CTA has tiles
+            const int mine = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+            for (int j = i; j < i + NST && j < mine; j++)
+                mbar_wait(&bar[ring_stage(j, NST)], ring_parity(j, NST), SPK_WAIT_ITERS);
         }
         __syncthreads();
     }

@@ -11,7 +11,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("kernel", ["line"])
+@pytest.mark.parametrize("kernel", ["line", "axis"])
 def test_drain_covers_the_loads_in_flight(kernel, tmp_path):
     if shutil.which("g++") is None:
         pytest.skip("g++ not available")
