@@ -343,15 +343,20 @@ int spk_spectrum(spk_ctx* ctx, int f1, int f2, double* out, int max_bins, int* n
  * counterpart: it reports on the B200 pipeline. */
 int spk_step_info(spk_ctx* ctx, int* kernels_per_step, double* bytes_per_step);
 
-/* Per-pass timing of one RK3 stage: each pass of stage 2 (no cleaning, no
- * dt reduction) is launched `reps` times between CUDA events on the context
- * stream.  out[i]: pass name, average ms per launch, algorithmic bytes per
- * launch, launches per step.  With deferred masked modes (HD/MHD RK3: the
- * RHS of stages 0-1 updates the kept modes only and stage 2 also moves the
- * modes outside the 2/3 mask once) the stage-2 RHS ("rhs_rk", once per step)
- * and the stage-1 RHS ("rhs_rk_01", twice) are reported apart.  The passes
- * update the context state (stage updates), so call it on a context whose
- * state may change.  No reference counterpart. */
+/* Per-pass timing of an RK3 step: each pass (no cleaning, no dt reduction) is
+ * launched `reps` times between CUDA events on the context stream.  out[i]:
+ * pass name, average ms per launch, algorithmic bytes per launch, launches
+ * per step; at most seven entries, each a pass that a step runs.  Passes that
+ * differ between the stages are timed as stage 2 runs them, and with deferred
+ * masked modes (HD/MHD RK3: stages 0-1 update the kept modes only and stage 2
+ * also moves the modes outside the 2/3 mask once) the stage-2 RHS ("rhs_rk",
+ * once per step) and what stages 0-1 run in its place are reported apart:
+ * the stage-1 RHS ("rhs_rk_01", twice), or where a step runs the x forward,
+ * the RHS and the next stage's x inverse of these stages as one kernel that
+ * kernel ("x_fwd_rhs_x_inv", twice; x_inverse is then stage 0's and x_forward
+ * stage 2's, once each).  The passes update the context state (stage
+ * updates), so call it on a context whose state may change.  No reference
+ * counterpart. */
 typedef struct spk_pass_stat {
     char   name[24];
     double ms;

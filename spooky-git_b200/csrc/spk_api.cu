@@ -2421,17 +2421,21 @@ extern "C" int spk_profile_passes(spk_ctx* c, int reps, spk_pass_stat_t* out, in
     }
     const PassBytes pb = pass_bytes(c, live);
     TrimScope ts(c);   // time the passes as a step runs them
-    // with deferred masked modes the RHS of stages 0-1 (kept modes) and of
-    // stage 2 (kept modes + the step's masked modes) are timed apart
-    // (rhs_rk_01 runs in a step only where the fused pass does not)
+    // With deferred masked modes the RHS of stages 0-1 (kept modes) and of
+    // stage 2 (kept modes + the step's masked modes) are timed apart.  Where a
+    // step runs stages 0 and 1 fused, its only x inverse is stage 0's, its x
+    // forward and RHS are stage 2's, and the fused pass takes the place of the
+    // stage-1 RHS: seven passes at most.
     const bool fused = xrhs_able(c);
-    const char* names[8] = {"x_inverse", "y_inverse", "z_products", "y_forward", "x_forward", "rhs_rk", "rhs_rk_01", "x_fwd_rhs_x_inv"};
-    const double bytes[8] = {pb.x_inv, pb.y_inv, pb.z, pb.y_fwd, pb.x_fwd, pb.rhs[2], pb.rhs[1], pb.xr};
-    const int per_step[8] = {fused ? 1 : 3, 3, 3, 3, fused ? 1 : 3, c->defer ? 1 : 3, fused ? 0 : 2, 2};
-    const int npass = fused ? 8 : (c->defer ? 7 : 6);
+    const int xi_stage = fused ? 0 : 2;
+    const char* names[7] = {"x_inverse", "y_inverse", "z_products", "y_forward", "x_forward", "rhs_rk",
+                            fused ? "x_fwd_rhs_x_inv" : "rhs_rk_01"};
+    const double bytes[7] = {pb.x_inv, pb.y_inv, pb.z, pb.y_fwd, pb.x_fwd, pb.rhs[2], fused ? pb.xr : pb.rhs[1]};
+    const int per_step[7] = {fused ? 1 : 3, 3, 3, 3, fused ? 1 : 3, c->defer ? 1 : 3, 2};
+    const int npass = c->defer ? 7 : 6;
     int n = 0;
     // one warm pipeline so every buffer holds stage data
-    pass_x_inverse(c, c->U, true, 2);
+    pass_x_inverse(c, c->U, true, xi_stage);
     pass_y_inverse(c, true);
     pass_z_products(c, false);
     pass_y_forward(c, c->nout, c->bufA, c->bufB);
@@ -2440,14 +2444,18 @@ extern "C" int spk_profile_passes(spk_ctx* c, int reps, spk_pass_stat_t* out, in
         CK(cudaEventRecord(e0, c->stream));
         for (int r = 0; r < reps; r++) {
             switch (k) {
-                case 0: pass_x_inverse(c, c->U, true, 2); break;
+                case 0: pass_x_inverse(c, c->U, true, xi_stage); break;
                 case 1: pass_y_inverse(c, true); break;
                 case 2: pass_z_products(c, false); break;
                 case 3: pass_y_forward(c, c->nout, c->bufA, c->bufB); break;
                 case 4: pass_x_forward(c); break;
                 case 5: { XfArgs x = xf_args(c, c->U, XM_RK2, false); rhs(c, x); } break;
-                case 6: { XfArgs x = xf_args(c, c->U, XM_RK1, false); rhs(c, x); } break;
-                default: { XfArgs x = xf_args(c, c->U, XM_RK1, false); xrhs(c, x); } break;
+                default: {
+                    XfArgs x = xf_args(c, c->U, XM_RK1, false);
+                    if (fused) xrhs(c, x);
+                    else rhs(c, x);
+                    break;
+                }
             }
         }
         CK(cudaEventRecord(e1, c->stream));

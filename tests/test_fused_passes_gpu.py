@@ -102,3 +102,33 @@ def test_line_pass_matches_oracle(ny, form):
     ctx.compute_dfield(Ud, dU)
     assert rel_l2(dU.cpu().numpy(), O.Oracle(p).compute_dfield(U)) < TOL_RHS[form]
 
+
+
+# the pass table names what a step runs: its launches add up to the step's
+# (less k_reset_max, k_dt and k_masked_rk) within the seven entries a caller
+# provides, and the kernels it times are the step's.  nx = 16 has no fused pass.
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("nx", [16, 32])
+def test_profiled_passes_are_those_of_a_step(nx, form):
+    import ctypes
+    from torch.profiler import ProfilerActivity, profile
+    from spooky_b200 import PassStat, lib
+    p = params((nx, 32, 32), 1, form)
+    ctx = Context(p)
+    ctx.set_state(state(p, 11, False))
+    ctx.advance(2)
+    ctx.synchronize()
+    out, n = (PassStat * 7)(), ctypes.c_int()
+
+    def kernels(call):
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            call()
+            ctx.synchronize()
+        return {e.name for e in prof.events() if "spk::" in e.name}
+
+    steps = kernels(lambda: ctx.advance(2))
+    timed = kernels(lambda: ctx._check(lib().spk_profile_passes(ctx._h, 1, out, 7, ctypes.byref(n))))
+    assert steps and timed and timed <= steps, timed - steps
+    table = {out[i].name.decode(): out[i].launches_per_step for i in range(n.value)}
+    assert sum(table.values()) == ctx.step_info()[0] - 3
+    assert ("x_fwd_rhs_x_inv" in table) == (nx == 32) and 0 not in table.values()
