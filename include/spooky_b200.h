@@ -567,7 +567,7 @@ int spk_trainer_train(spk_trainer* tr, int nsteps, int batch, float lr, float* l
 
 /* Schedule autotuner (no reference counterpart).  Picks, by timing whole
  * recorded steps with CUDA events, the launch choices that leave the
- * arithmetic unchanged: the axis tile width of short axes, the z pass's
+ * arithmetic unchanged: the x inverse's tile width at short lengths, the z pass's
  * lines per CTA, the axis passes' pipeline stages and the RHS grid (CTAs
  * per SM), by coordinate descent
  * over candidate values; the tuned context computes the same bits as an
@@ -581,11 +581,17 @@ int spk_autotune(spk_ctx* ctx, int steps, int* z_lines, int* axis_stages, int* r
 /* The same for every group of an ensemble (each group tuned on its own). */
 int spk_ensemble_autotune(spk_ensemble* ens, int steps);
 /* The context's launch schedule: the three knobs above (0: the launcher's
- * own model) and the axis tile divisor -- 2 gives the axis passes of axes up
- * to 64 long half-width tiles (a 64^3 box has 33 kz columns, 21 below the
- * 2/3 cut-off, in a 64-column tile), 1 the full tiles; the autotuner tries
- * both where an axis is that short.  Setting it (e.g. a schedule tuned on
- * another context of the same grid) re-records the step graph; the values
+ * own model) and the axis tile divisor.  Each is a request that the launches
+ * it concerns follow where they can: z_lines that do not fit shared memory or
+ * do not divide an ensemble box's lines leave the launcher its own choice,
+ * and an odd number is rounded up where an odd number of channels pairs
+ * its lines (HD); axis_stages are 2 to 4 in the passes whose transforms a
+ * warp owns (1 leaves them their own choice) and not used by the fused stage
+ * pass; axis_tile_div 2 gives the x inverse that reads the state half-width
+ * tiles at x lengths of 32 to 64 (a 64^3 box has 33 kz columns, 21 below the
+ * 2/3 cut-off), 1 the full tiles, and the autotuner tries both there.
+ * spk_get_schedule returns the requests.  Setting it (e.g. a schedule tuned
+ * on another context of the same grid) re-records the step graph; the values
  * computed do not change. */
 int spk_get_schedule(const spk_ctx* ctx, int* z_lines, int* axis_stages, int* rhs_ctas_per_sm, int* axis_tile_div);
 int spk_set_schedule(spk_ctx* ctx, int z_lines, int axis_stages, int rhs_ctas_per_sm, int axis_tile_div);

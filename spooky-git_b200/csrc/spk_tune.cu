@@ -6,11 +6,15 @@
 // a tuned context computes the same values as an untuned one:
 //   tune_zl   lines per CTA of the z pass (shared memory per CTA against the
 //             busy transform slots: the launcher's own choice is a model);
+//             an odd number is rounded up where an odd channel pairs its
+//             lines (HD);
 //   tune_nst  pipeline stages of the axis passes (TMA loads in flight against
-//             CTAs per SM);
+//             CTAs per SM); k_line has 2 to 4, k_xrhs one set of tiles;
 //   tune_rhs  CTAs per SM of the RHS grid (loads in flight against tail);
-//   tune_kt   half-width tiles for the axis passes of axes up to 64 long
-//             (fewer idle columns against fewer threads per CTA).
+//   tune_kt   half-width k_axis2 tiles (fewer idle columns against fewer
+//             threads per CTA): of the x inverse from the state at x lengths
+//             of 32 to 64.  Shorter tiles would not fill a warp, and the
+//             passes between buffers of these lengths are k_line's.
 // Coordinate descent over the knobs, each candidate timed with CUDA events
 // over whole recorded steps; the state and the step scalars are restored
 // afterwards.
@@ -53,7 +57,7 @@ extern "C" int spk_autotune(spk_ctx* c, int steps, int* zl, int* nst, int* rhs, 
     float best_ms = base;
     struct Knob { int* v; std::vector<int> cand; };
     // the tile width first: the stage count depends on it
-    const bool short_axis = c->nx <= 64 || c->ny <= 64;
+    const bool short_axis = c->nx >= 32 && c->nx <= 64;
     Knob knobs[4] = {{&c->tune_kt, short_axis ? std::vector<int>{0, 2} : std::vector<int>{}},
                      {&c->tune_zl, {1, 2, 4, 8, 16, 32, 64}}, {&c->tune_nst, {1, 2, 3, 4}}, {&c->tune_rhs, {6, 12, 24, 48}}};
     for (int kq = 0; kq < 4 && !rc; kq++) {

@@ -164,9 +164,10 @@ def _short_params(n, form, kind):
 def test_half_width_axis_tiles_compute_the_same_bits(kind, n, form):
     """The autotuner's half-width axis tiles of short axes (spk_set_schedule
     axis_tile_div 2) transform the same columns as the full tiles: the
-    same state after steps that use every axis pass (inverse passes with
-    derivatives, forward passes, the RKL2 flux chain of anisotropic
-    conduction)."""
+    same state after steps.  The knob reaches the x inverse that reads the
+    state at 32, 48 and 64 points, with theta's derivative and in the RKL2 flux
+    chain; the passes between buffers have tiles of their own, and a half tile
+    of 16 or 24 points would not fill a warp."""
     p = _short_params(n, form, kind)
     U = initial_state(p, 13)
     a, b = Context(p), Context(p)
