@@ -52,12 +52,14 @@ def check_steps(p, U, nsteps, tol):
     assert rel_l2(ctx.get_state(), o.get_state()) < tol
 
 
-# every x length k_xrhs covers; 24 y rows and 9 kz columns leave ragged tiles
+# every x length k_xrhs covers (24 in the FP32 form only: the plain form runs
+# k_axis2 there); 24 y rows and 9 kz columns leave ragged tiles
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("outside", [False, True])
+@pytest.mark.parametrize("mhd", [0, 1])
 @pytest.mark.parametrize("nx", [24, 32, 48, 64, 96, 128, 192, 256])
-def test_fused_stage_matches_oracle(nx, outside, form):
-    p = params((nx, 24, 16), nx % 3 == 0 or nx >= 128, form)
+def test_fused_stage_matches_oracle(nx, mhd, outside, form):
+    p = params((nx, 24, 16), mhd, form)
     check_steps(p, state(p, 5, outside), 3, TOL_STEP[form])
 
 
@@ -89,7 +91,8 @@ def test_fused_stage_mixed_group(form):
         assert rel_l2(b.get_state(), o.get_state()) < TOL_STEP[form]
 
 
-# every length k_line covers along y, with more than one k block
+# every length k_line covers along y (24 in the FP32 form only, 384 in the
+# plain form only: k_axis2 runs the other form there), with more than one k block
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("ny", [24, 32, 48, 64, 96, 128, 192, 256, 384])
 def test_line_pass_matches_oracle(ny, form):
@@ -103,6 +106,59 @@ def test_line_pass_matches_oracle(ny, form):
     assert rel_l2(dU.cpu().numpy(), O.Oracle(p).compute_dfield(U)) < TOL_RHS[form]
 
 
+# the same lengths where the y inverse loads the kept rows alone (a prefix and
+# a suffix from a multiple of 8) and the x forward filters its outer rows: steps
+# from a state inside the mask
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("ny", [24, 32, 48, 64, 96, 128, 192, 256, 384])
+def test_trimmed_line_pass_matches_oracle(ny, form):
+    p = params((32, ny, 48), 1, form)
+    check_steps(p, state(p, 10, False), 2, TOL_STEP[form])
+
+
+# HD: the odd channel (3 in, 5 out) pairs with itself on the next line of a
+# z-pass CTA, in the products and in to_real; from one lane to several warps a
+# transform, 48 lines (the last CTA may have fewer)
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("nz", [8, 32, 96, 256, 512, 768, 1024])
+def test_odd_channel_pairs_match_oracle(nz, form):
+    import torch
+    p = params((6, 8, nz), 0, form)
+    U = state(p, 12, True)
+    ctx = Context(p)
+    Ud = torch.from_numpy(U).cuda()
+    dU = torch.zeros_like(Ud)
+    ctx.compute_dfield(Ud, dU)
+    assert rel_l2(dU.cpu().numpy(), O.Oracle(p).compute_dfield(U)) < TOL_RHS[form]
+    check_steps(p, U, 2, TOL_STEP[form])
+    o = O.Oracle(p)
+    o.set_state(U)
+    ctx.set_state(U)
+    R = torch.zeros(ctx.shape_r, dtype=torch.float64, device="cuda")
+    ctx.to_real(R)
+    ctx.synchronize()
+    assert rel_l2(R.cpu().numpy(), o.to_real()) < (1e-13 if form == SPK_FORM_PLAIN else 1e-6)
+
+
+# the schedule leaves the values alone: lines per z-pass CTA (HD pairs lines,
+# so an odd number is rounded up) and stages of the axis passes
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("shape", [(24, 24, 32), (48, 64, 16), (96, 32, 256), (32, 128, 16), (256, 192, 8)])
+def test_schedule_keeps_the_bits(shape, form):
+    p = params(shape, 0, form)
+    U = state(p, 13, False)
+
+    def run(**knobs):
+        ctx = Context(p)
+        ctx.set_schedule(**knobs)
+        ctx.set_state(U)
+        ctx.advance(2)
+        ctx.synchronize()
+        return ctx.get_state()
+
+    ref = run()
+    for knobs in [dict(z_lines=n) for n in (1, 2, 3, 4, 8)] + [dict(axis_stages=n) for n in (1, 2, 3, 4)]:
+        assert np.array_equal(run(**knobs), ref), knobs
 
 # the pass table names what a step runs: its launches add up to the step's
 # (less k_reset_max, k_dt and k_masked_rk) within the seven entries a caller
