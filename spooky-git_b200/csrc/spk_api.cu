@@ -76,7 +76,7 @@ struct spk_ctx {
     // schedule knobs picked by spk_autotune (0: the launchers' own choice)
     int tune_zl = 0;               // z pass: lines per CTA
     int tune_nst = 0;              // axis passes: pipeline stages
-    int tune_kt = 0;               // axis passes of short axes: 2 = half-width tiles
+    int tune_kt = 0;               // x inverse of the state at short lengths: 2 = half-width tiles
     int tune_rhs = 0;              // RHS: CTAs per SM
     int ch_dx = -1, ch_dy = -1, ncl_half = 0;
     int ngrad = 0;                 // closure variant 2: gradient channels (9 or 18) from ch_dx
@@ -365,11 +365,12 @@ static void launch_axis_conv(spk_ctx* c, AxisArgs& a, long total) {
     if constexpr (sizeof(T) == 4 && DIR > 0) {
         if (a.convert) { launch_axis_ln<T, N, DIR, true>(c, a, total); return; }
     }
-    // k_line takes every forward pass of the lengths it covers
-    if constexpr (DIR > 0 || !line_ok<T, N, 128>()) {
+    // k_line takes every pass between buffers of the lengths it covers; what
+    // is left of them is the FP64 x inverse, whose input is the state
+    if constexpr ((DIR > 0 && sizeof(T) == 8) || !line_ok<T, N, 128>()) {
         launch_axis_ln<T, N, DIR, false>(c, a, total);
     } else {
-        c->err = "internal: a forward axis pass without its kernel";
+        c->err = "internal: an axis pass without its kernel";
         c->sticky = SPK_ERR_CUDA;
     }
 }
