@@ -126,9 +126,9 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
                         a.axis == 0 ? row : x.o, ch);
         }
     };
-    auto issue = [&](int t, int s) {   // the group's first thread
+    auto issue = [&](int t, int s, int j) {   // load j of the group, by its first thread
+        *issued = j + 1;
         const Where x = where(t);
-        ++*issued;
         if (x.skip) { mbar_expect_tx(&bar[s], 0); return; }
         const LineSeg* seg = x.clear ? a.in_trim : a.in;
         mbar_expect_tx(&bar[s], (uint32_t)((seg[0].rows * seg[0].n + seg[1].rows * seg[1].n) * 128));
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
         for (int s = 0; s < nst; s++) { mbar_init(&bar[s], 1); mbar_init(&empty[s], W); }
         fence_mbar_init();
         for (int s = 0; s < nst; s++)
-            if (first + s * step < total) issue(first + s * step, s);
+            if (first + s * step < total) issue(first + s * step, s, s);
     }
     regfft_fill_twiddles<T, N>(tw, (const C2<T>*)a.plan.tw, tid, blockDim.x);
     for (int i = tid; i < N; i += blockDim.x) kax[i] = (T)(a.axis == 0 ? a.g.kx : a.g.ky)[i];
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(LineCfg<T, N>::WARPS * 32, LineCfg<T, N>::MINB
                 else dead = !mbar_wait(&empty[sp], (uint32_t)(((it - 1) / nst) & 1), SPK_WAIT_ITERS);
                 if (!dead) {
                     fence_proxy_async_smem();
-                    issue(tn, sp);
+                    issue(tn, sp, it + nst - 1);
                 }
             }
         };

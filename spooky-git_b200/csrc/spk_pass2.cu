@@ -318,8 +318,7 @@ __global__ void __launch_bounds__(256, axis_minb<T, N>()) k_axis2(const __grid_c
         if (tid == 0) {
             atomicExch(a.err, 2);
             // bounded drain: the loads of tiles i .. i + NST - 1, as far as this CTA has tiles
-            const int mine = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-            for (int j = i; j < i + NST && j < mine; j++)
+            for (int j = i; j < i + NST && (int)blockIdx.x + j * (int)gridDim.x < total; j++)
                 mbar_wait(&bar[ring_stage(j, NST)], ring_parity(j, NST), SPK_WAIT_ITERS);
         }
         __syncthreads();
