@@ -6,7 +6,7 @@
 // tile, 16 warps, 38-43% of issue slots, 51-69% of the copy bandwidth).
 // Here a tile of 128-byte rows is loaded by TMA (swizzled) and transformed in
 // place by the warps that own its columns: no exchange buffer, 24 warps per
-// SM, one barrier of the tile's warps per tile.  The inverse, which writes
+// SM (16 for the FP64 lengths 3 2^k), one barrier of the tile's warps per tile.  The inverse, which writes
 // every row, stores the tile by TMA; the forward passes, which write the kept
 // rows, copy them out in 16-byte pieces (TMA boxes of the kept rows measured
 // 0.149 ms at 256^3 FP32, the copy 0.141).  Loads take the rows and columns
@@ -17,7 +17,10 @@
 //   128^3 FP32  0.029 0.027 0.021 -> 0.021 0.019 0.015
 //   64^3  FP32  0.012 0.011 0.011 -> 0.009 0.008 0.008
 // At 256^3 both directions wait for memory (long-scoreboard stalls of the
-// tile waits, 4.8-5.3 TB/s moved); refilling a stage before the next tile's
+// tile waits, 4.5-4.9 TB/s moved, 51-55% of issue slots).  The FP32 forward
+// passes of 256 points gain nothing by themselves, but the step is no slower
+// with them (four steps 10.286 ms, 10.287 with k_axis2's) and other lengths
+// are faster (192^3 5.82 ms against 6.11): one rule for all.  Refilling a stage before the next tile's
 // wait, more tiles of fewer warps, and L2 promotion of 64 to 256 bytes
 // measured no better.
 //

@@ -360,8 +360,9 @@ __host__ __device__ inline bool zpass_alias(int gen, int nstages, int ninv, int 
 // own, or with xline pairs with the same channel of the next line (the last
 // line of an odd number stays alone).  HD makes 4 transforms a line that way
 // (3 channels in, 5 out) instead of 5: 512^3 FP32 2.56 -> 2.05 ms a pass,
-// 256^3 FP32 0.256 -> 0.213, FP64 0.533 -> 0.433.  Boussinesq contexts keep the pairs within the line: the conduction
-// cycle carries a changed FP32 rounding through every stage after it.
+// 256^3 FP32 0.256 -> 0.213, FP64 0.533 -> 0.433.  Boussinesq contexts, one rule
+// for all of them, keep the pairs within the line: the conduction cycle that
+// they may run carries a changed FP32 rounding through every stage after it.
 __host__ __device__ inline int zpass_pairs(int nch, int lines, int xline) {
     return (nch / 2) * lines + ((nch & 1) ? (xline ? (lines + 1) / 2 : lines) : 0);
 }
@@ -924,8 +925,9 @@ __device__ __forceinline__ double2 rk_value(const XfArgs& a, size_t gi, double2 
         case XM_RK1: {
             // the scheme's S = U2 + x1 dt R has x1 = -g1, so it is the S that
             // was read, but for rounding: the store (one array of the stage's
-            // four) is left out.  Boussinesq contexts keep it: their conduction
-            // cycle carries a last bit of the state through every FP32 stage.
+            // four) is left out.  Boussinesq contexts keep it, one rule for all of
+            // them: the conduction cycle that they may run carries a last bit
+            // of the state through every FP32 stage.
             const double bu = g1 * dt, bs = x1 * dt;
             const double2 Un = d2(1.0 * S.x + bu * R.x, 1.0 * S.y + bu * R.y);
             if (a.bous) a.S[gi] = d2(1.0 * Un.x + bs * R.x, 1.0 * Un.y + bs * R.y);

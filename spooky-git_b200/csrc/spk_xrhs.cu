@@ -13,16 +13,17 @@
 //   4. x inverse of the three fields, TMA stores to the pass buffer.
 // As separate passes the products and the new state each made a round trip
 // through HBM: at 256^3 MHD, FP32, 2.0 GB per stage and 0.37 ms (x forward
-// 0.096, RHS 0.158, x inverse 0.112) against 1.1 GB and 0.29 ms here; the step
+// 0.096, RHS 0.158, x inverse 0.112) against 1.1 GB and 0.27 ms here; the step
 // goes from 2.75 to 2.59 ms, plain 5.04 to 4.87, 64^3 FP32 0.134 to 0.115
 // (two launches fewer a stage).
 // The pass is bound by latency: 64-byte rows keep five channels of N = 256
 // within 80 KB, so two CTAs of 256 threads (128 registers) share an SM and
 // overlap their phases.  Prefetching the state's rows into L2 while the
-// products arrive measured slower (by TMA 0.309 ms, per thread 0.316), and so
-// did loading the products by cp.async (0.314).  Half of a tile's time goes to
-// step 3, whose rows lie in 45 pages per array: the loads of one mode ahead
-// cover part of their latency.
+// products arrive measured slower (four steps 10.42 ms without, 10.56 by TMA,
+// 10.60 per thread), and so did loading the products by cp.async (10.59).
+// Three fifths of a tile's time go to step 3 (phase clocks at 256^3 FP32: 23k
+// of 39k cycles), whose rows lie in 45 pages per array: the loads of one mode
+// ahead cover part of their latency.
 //
 // Boxes with masked content (DevScalars::masked_live) walk every (ky, kz)
 // tile: their masked modes enter the inverse scaled to the next stage, as in
